@@ -133,10 +133,7 @@ __device__ __forceinline__ void right_mult(Link<R> &L, const R h[4])
 }
 
 // ---- Philox4x32-10 (Salmon, Moraes, Dror, Shaw, SC'11) ---------------------------------------
-// Not inlined: a heat-bath site update draws from up to eight call sites per subgroup, three
-// subgroups per update, and inlined copies of the ten rounds made the kernel's code outgrow the
-// instruction cache (the SA pass stalled on instruction fetch more than on anything else).
-static __device__ __noinline__ uint4 philox4x32_10(uint4 c, uint2 k)
+__device__ __forceinline__ uint4 philox4x32_10_inline(uint4 c, uint2 k)
 {
 #pragma unroll
     for (int r = 0; r < 10; r++) {
@@ -150,6 +147,9 @@ static __device__ __noinline__ uint4 philox4x32_10(uint4 c, uint2 k)
     }
     return c;
 }
+// Out of line for the draws off the common path and the rules that draw at several places: copies of
+// the ten rounds at each of them make a kernel's code outgrow the instruction cache.
+static __device__ __noinline__ uint4 philox4x32_10(uint4 c, uint2 k) { return philox4x32_10_inline(c, k); }
 
 // The reference's per-thread generator (lattice/rng/PhiloxWrapper.hxx:92-137): key = (tid, seed),
 // counter = (k, launch counter, 0x12345678, 0xabcdef09), the k = 0 block discarded; floats are
@@ -160,11 +160,13 @@ struct Rng {
     uint4 ctr;
     uint4 res;
     int local;
+    uint32_t drawn;  // numbers drawn so far, for the heat bath, which addresses its draws by index
     __device__ __forceinline__ void init(uint32_t tid, uint32_t seed, uint32_t counter)
     {
         key = make_uint2(tid, seed);
         ctr = make_uint4(0u, counter, 0x12345678u, 0xabcdef09u);
         local = 0;
+        drawn = 0;
     }
     __device__ __forceinline__ R rand();
 };
@@ -261,18 +263,268 @@ __device__ __forceinline__ void upd_micro(R a[4])
     a[3] *= b;
 }
 
-// Kennedy-Pendleton heat-bath, SaUpdate::calculateUpdate (SaUpdate.hxx:103-146).  The literal
-// types follow the reference (double constants, cospi of a double argument), so the FP32
-// variant promotes where the reference promotes.  Every rejection loop is bounded (2^16 draws).
-// The inner loops accept with probability >= 0.9999 per draw; the outer one accepts rarely when
-// p0 = T/|a| is large (a site whose subgroup coupling |a| is tiny against the temperature), and
-// there the reference would keep drawing.  Such a site -- the outer bound exhausted, or |a| = 0
-// -- takes a0 from the p0 -> infinity limit of the same distribution, the Haar measure (density
-// proportional to sqrt(1 - a0^2), sampled by rejection), instead of the unaccepted 1 - delta,
-// whose square root below would be NaN for delta > 2.
+// ---- heat bath ---------------------------------------------------------------------------------
+// Number n (0, 1, 2, ...) of a site's stream is word pair / word 3 - n % 4 (doubles: the upper, then
+// the lower half) of Philox block 1 + n / (numbers per block), so any lane can draw any number.
+__device__ __forceinline__ float draw_word(const uint4 &b, uint32_t j, float)
+{
+    const uint32_t v = j == 0 ? b.w : (j == 1 ? b.z : (j == 2 ? b.y : b.x));
+    return (float)(1u + (v >> 8)) * 0x1.fffffep-25f;
+}
+__device__ __forceinline__ double draw_word(const uint4 &b, uint32_t j, double)
+{
+    const uint64_t v = j == 0 ? (((uint64_t)b.w << 32) | b.z) : (((uint64_t)b.y << 32) | b.x);
+    return (double)(1ull + (v >> 11)) * 0x1.fffffffffffffp-54;
+}
 template <typename R>
+struct PerBlock {
+    static constexpr uint32_t log2 = sizeof(R) == 4 ? 2 : 1, mask = (1u << log2) - 1u;
+};
+
+// HOT: with the rounds in line.  The two-lane layout has one copy of the heat bath and gains from it
+// (32^4, FP32 Landau / U1xU1: 146 / 234 us per pass against 150 / 258 us); the four-lane layout has
+// three and waits for instructions then.
+template <typename R, bool HOT = false>
+__device__ __forceinline__ uint4 draw_block(uint2 key, uint32_t counter, uint32_t n)
+{
+    const uint4 c = make_uint4(1u + (n >> PerBlock<R>::log2), counter, 0x12345678u, 0xabcdef09u);
+    return HOT ? philox4x32_10_inline(c, key) : philox4x32_10(c, key);
+}
+template <typename R>
+__device__ __forceinline__ R draw_at(uint2 key, uint32_t counter, uint32_t n)
+{
+    return draw_word(draw_block<R>(key, counter, n), n & PerBlock<R>::mask, R());
+}
+
+// numbers n and n + 1; usually in one block
+template <typename R, bool HOT = false>
+__device__ __forceinline__ void draw_two(uint2 key, uint32_t counter, uint32_t n, R u[2])
+{
+    const uint4 b = draw_block<R, HOT>(key, counter, n);
+    const uint32_t j = n & PerBlock<R>::mask;
+    u[0] = draw_word(b, j, R());
+    u[1] = j == PerBlock<R>::mask ? draw_at<R>(key, counter, n + 1) : draw_word(b, j + 1, R());
+}
+
+// numbers n .. n + 3: one or two blocks of floats, two (three for odd n) of doubles
+template <bool HOT>
+__device__ __forceinline__ void draw_four(uint2 key, uint32_t counter, uint32_t n, float u[4])
+{
+    const uint4 b = draw_block<float, HOT>(key, counter, n);
+    const uint32_t j = n & 3u;
+    uint4 c = b;
+    if (j) c = draw_block<float>(key, counter, n + 4);
+#pragma unroll
+    for (uint32_t k = 0; k < 4; k++) u[k] = j + k < 4 ? draw_word(b, j + k, 0.f) : draw_word(c, j + k - 4, 0.f);
+}
+template <bool HOT>
+__device__ __forceinline__ void draw_four(uint2 key, uint32_t counter, uint32_t n, double u[4])
+{
+    draw_two<double, HOT>(key, counter, n, u);
+    draw_two<double, HOT>(key, counter, n + 2, u + 2);
+}
+
+// One trial of the Kennedy-Pendleton rejection loop, its draws starting at number n (SaUpdate.hxx:
+// 103-128).  The literal types follow the reference (double constants, cospi of a double argument),
+// so the FP32 variant promotes where the reference promotes.  Returns the acceptance; `used` is the
+// number of draws, 4 unless a number below 0.0001 was drawn again (2e-4 of the trials).
+template <typename R, bool HOT>
+__device__ __forceinline__ bool kp_trial(uint2 key, uint32_t counter, uint32_t n, R p0, R &delta, uint32_t &used)
+{
+    R u[4];
+    draw_four<HOT>(key, counter, n, u);
+    used = 4;
+    if (u[0] < 0.0001 || u[1] < 0.0001) {
+        uint32_t q = n;
+        int g1 = 0, g2 = 0;
+        do { u[0] = draw_at<R>(key, counter, q++); } while (u[0] < 0.0001 && ++g1 < 65536);
+        do { u[1] = draw_at<R>(key, counter, q++); } while (u[1] < 0.0001 && ++g2 < 65536);
+        u[2] = draw_at<R>(key, counter, q++);
+        u[3] = draw_at<R>(key, counter, q++);
+        used = q - n;
+    }
+    const R r1 = -lg(u[0]) * p0;
+    const R r2 = -lg(u[1]) * p0;
+    R r3 = (R)cospi(2.0 * (double)u[2]);
+    r3 = r3 * r3;
+    delta = r2 + r1 * r3;
+    const R r4 = u[3];
+    return !(r4 * r4 > (1.0 - 0.5 * delta));
+}
+
+// position of set bit number g (0-based) of mask, g < popc(mask)
+__device__ __forceinline__ int nth_bit(uint32_t mask, int g)
+{
+    int pos = 0;
+#pragma unroll
+    for (int w = 16; w > 0; w >>= 1) {
+        const int c = __popc((mask >> pos) & ((1u << w) - 1u));
+        if (g >= c) {
+            g -= c;
+            pos += w;
+        }
+    }
+    return pos;
+}
+
+constexpr uint32_t kMaxTrials = 65536;  // bound of a site's rejection loop
+constexpr int kScreenRound = 8;         // rounds of shared trials before the sites left are screened
+
+// The rest of the loop of one site, all arguments the same in every lane: rows of 32 trials, four at
+// a time.  delta >= r2 = -ln(u1) p0, and delta > 2 is never accepted, so where p0 is large nearly
+// every trial is decided by its second number alone: u1 < exp(-2 / p0) (less a margin that covers
+// the rounding of r2) and neither of the first two numbers drawn again.  Only the other trials are
+// evaluated, in order.  Such a site often runs into the bound, 2048 rows.
+template <typename R, bool HOT>
+__device__ __forceinline__ bool kp_screened(uint2 key, uint32_t counter, R p0, R &delta, uint32_t &n, uint32_t &trials)
+{
+    constexpr uint32_t full = 0xffffffffu;
+    constexpr int rows = 4;
+    const int lane = threadIdx.x & 31;
+    const float bar = p0 > (R)1 && p0 < (R)1e30 ? expf(-2.f / (float)p0) - 1e-5f : 0.f;
+    while (trials < kMaxTrials) {
+        uint32_t open[rows];
+#pragma unroll
+        for (int q = 0; q < rows; q++) {
+            const uint32_t k = 32u * q + lane;
+            R u[2];
+            draw_two<R, HOT>(key, counter, n + 4u * k, u);
+            const bool rejected = !(u[0] < 0.0001) && !(u[1] < 0.0001) && (float)u[1] < bar;
+            open[q] = __ballot_sync(full, !rejected && trials + k < kMaxTrials);
+        }
+        uint32_t steps = min(32u * rows, kMaxTrials - trials), drawn = 4u * steps;
+        bool accepted = false, ended = false;
+#pragma unroll 1
+        for (int q = 0; q < rows && !ended; q++) {
+            const uint32_t row = q == 0 ? open[0] : (q == 1 ? open[1] : (q == 2 ? open[2] : open[3]));
+            if (!row) continue;
+            R d = 0;
+            uint32_t used = 4;
+            bool acc = false;
+            if ((row >> lane) & 1u) acc = kp_trial<R, HOT>(key, counter, n + 4u * (32u * q + lane), p0, d, used);
+            const uint32_t ends = __ballot_sync(full, acc || used != 4);
+            if (!ends) continue;
+            const int f = __ffs(ends) - 1;
+            ended = true;
+            accepted = __shfl_sync(full, (int)acc, f);
+            delta = __shfl_sync(full, d, f);
+            steps = 32u * q + f + 1;
+            drawn = 4u * (steps - 1) + __shfl_sync(full, used, f);
+        }
+        n += drawn;
+        trials += steps;
+        if (accepted) return true;
+    }
+    return false;
+}
+
+// The rejection loops of the S sites of a warp (site lane & (S - 1)), all 32 lanes together.  A
+// site's trials are independent given where their draws start, and trial k starts 4 draws after trial
+// k - 1 unless that one drew a number again.  So the lanes evaluate consecutive trials of the sites
+// still looping, 32 / (such sites) each, and every site takes its first accepted trial; a trial that
+// drew again ends the run of known starts, and the site goes on behind it.  The result is what one
+// lane per site computes, draw for draw, but a warp loops for its total number of trials over 32
+// instead of its slowest site's number.
+// pending: this lane's site wants a trial.  Returns whether a trial was accepted within the bound;
+// delta and n (draws used so far) are updated.
+template <typename R, int S>
+__device__ __forceinline__ bool kp_warp(bool pending, uint2 key, uint32_t counter, R p0, R &delta, uint32_t &n)
+{
+    static_assert(S == 8 || S == 16, "four or two lanes per site");
+    constexpr uint32_t full = 0xffffffffu, sites = (1u << S) - 1u;
+    const int lane = threadIdx.x & 31, site = lane & (S - 1);
+    bool accepted = false;
+    uint32_t trials = 0;
+    uint32_t need = __ballot_sync(full, pending) & sites;
+    for (int round = 0; need && round < kScreenRound; round++) {
+        // this lane's trial: number m of the site whose draws these are.  In the first round every site
+        // takes its own lanes; after it the lanes are shared out again.
+        R ps = p0;
+        uint2 ks = key;
+        uint32_t cs = counter, ns = n, ts = trials;
+        int m = lane / S, shift = 0;
+        bool active = pending;
+        if (round > 0) {
+            const int count = __popc(need);
+            shift = __clz(count - 1) - 27;  // 32 >> ceil(log2 count) lanes for each of them
+            const int mine = lane >> shift, src = nth_bit(need, mine < count ? mine : 0);
+            m = lane & ((1 << shift) - 1);
+            ps = __shfl_sync(full, p0, src);
+            ks = make_uint2(__shfl_sync(full, key.x, src), __shfl_sync(full, key.y, src));
+            cs = __shfl_sync(full, counter, src);
+            ns = __shfl_sync(full, n, src);
+            ts = __shfl_sync(full, trials, src);
+            active = mine < count && ts + m < kMaxTrials;
+        }
+        R d = 0;
+        uint32_t used = 4;
+        bool acc = false;
+        if (active) acc = kp_trial<R, S == 16>(ks, cs, ns + 4u * m, ps, d, used);
+        const uint32_t accs = __ballot_sync(full, acc), again = __ballot_sync(full, used != 4), ends = accs | again;
+        // the first trial of this lane's site that ends its run, and the lane that evaluated it
+        uint32_t seg, per;
+        int first, from;
+        if (round > 0) {
+            const int base = (__popc(need & ((1u << site) - 1u)) << shift) & 31;  // (sites done: any lane)
+            per = 1u << shift;
+            seg = (ends >> base) & (per == 32 ? full : (1u << per) - 1u);
+            first = seg ? __ffs(seg) - 1 : 0;
+            from = base + first;
+        } else {
+            per = 32 / S;
+            seg = (ends >> site) & (S == 16 ? 0x00010001u : 0x01010101u);
+            const int bit = seg ? __ffs(seg) - 1 : 0;
+            first = bit / S;
+            from = site + bit;
+        }
+        const R df = __shfl_sync(full, d, from);
+        const uint32_t uf = again ? __shfl_sync(full, used, from) : 4u;
+        if (pending) {
+            if (seg) {
+                n += 4u * first + uf;
+                trials += first + 1;
+                if ((accs >> from) & 1u) {
+                    accepted = true;
+                    delta = df;
+                }
+            } else {
+                const uint32_t done = min(per, kMaxTrials - trials);
+                n += 4u * done;
+                trials += done;
+            }
+            pending = !accepted && trials < kMaxTrials;
+        }
+        need = __ballot_sync(full, pending) & sites;
+    }
+    while (need) {
+        const int src = __ffs(need) - 1;
+        need &= need - 1;
+        R d = 0;
+        uint32_t ns = __shfl_sync(full, n, src), ts = __shfl_sync(full, trials, src);
+        const bool acc = kp_screened<R, S == 16>(make_uint2(__shfl_sync(full, key.x, src), __shfl_sync(full, key.y, src)),
+                                        __shfl_sync(full, counter, src), __shfl_sync(full, p0, src), d, ns, ts);
+        if (site == src) {
+            n = ns;
+            accepted = acc;
+            delta = d;
+        }
+    }
+    return accepted;
+}
+
+// Kennedy-Pendleton heat bath, SaUpdate::calculateUpdate (SaUpdate.hxx:103-146), by all lanes of a
+// warp that holds S sites.  A site's loop is bounded (2^16 trials): its acceptance is rare when
+// p0 = T/|a| is large (a subgroup coupling |a| tiny against the temperature), and there the
+// reference would keep drawing.  Such a site -- the bound exhausted, or |a| = 0 -- takes a0 from the
+// p0 -> infinity limit of the same distribution, the Haar measure (density proportional to
+// sqrt(1 - a0^2), sampled by rejection), instead of the unaccepted 1 - delta, whose square root below
+// would be NaN for delta > 2.
+template <typename R, int S>
 __device__ __forceinline__ void upd_sa(R a[4], float temperature, Rng<R> &rng)
 {
+    const uint2 key = rng.key;
+    const uint32_t counter = rng.ctr.y;
+    uint32_t n = rng.drawn;
     R e0 = a[0], e1 = -a[1], e2 = -a[2], e3 = -a[3];
     const R nrm2 = e0 * e0 + e1 * e1 + e2 * e2 + e3 * e3;
     const bool flat = !(nrm2 > (R)0);  // no coupling: the local distribution is Haar
@@ -281,36 +533,25 @@ __device__ __forceinline__ void upd_sa(R a[4], float temperature, Rng<R> &rng)
         e0 = 1;
         e1 = e2 = e3 = 0;
     }
-    const R p0 = dk * temperature;
-    R r1, r2, r3, r4, delta = 0;
-    bool accepted = false;
-    int guard = 0;
-    if (!flat) {
-        do {
-            int g1 = 0, g2 = 0;
-            do { r1 = rng.rand(); } while (r1 < 0.0001 && ++g1 < 65536);
-            r1 = -lg(r1) * p0;
-            do { r2 = rng.rand(); } while (r2 < 0.0001 && ++g2 < 65536);
-            r2 = -lg(r2) * p0;
-            r3 = (R)cospi(2.0 * (double)rng.rand());
-            r3 = r3 * r3;
-            delta = r2 + r1 * r3;
-            r4 = rng.rand();
-            accepted = !(r4 * r4 > (1.0 - 0.5 * delta));
-        } while (!accepted && ++guard < 65536);
-    }
+    R delta = 0;
+    const bool accepted = kp_warp<R, S>(!flat, key, counter, dk * temperature, delta, n);
     R a0 = (R)(1.0 - delta);
     if (!accepted) {
         int g = 0;
+        R r4;
         do {
-            a0 = (R)(2.0 * rng.rand() - 1.0);
-            r4 = rng.rand();
+            a0 = (R)(2.0 * draw_at<R>(key, counter, n) - 1.0);
+            r4 = draw_at<R>(key, counter, n + 1);
+            n += 2;
         } while (r4 * r4 > (R)1 - a0 * a0 && ++g < 64);
     }
-    const R cos_theta = (R)(2.0 * rng.rand() - 1.0);
+    R u[2];
+    draw_two<R, S == 16>(key, counter, n, u);
+    rng.drawn = n + 2;
+    const R cos_theta = (R)(2.0 * u[0] - 1.0);
     const R sin_theta = (R)sqrt(1.0 - (double)(cos_theta * cos_theta));
     const R sin_alpha = sq((R)(1 - a0 * a0));
-    const R phi = (R)(2.0 * rng.rand());
+    const R phi = (R)(2.0 * u[1]);
     const R a1 = sin_alpha * sin_theta * cpi(phi);
     const R a2 = sin_alpha * sin_theta * spi(phi);
     const R a3 = sin_alpha * cos_theta;
@@ -358,13 +599,15 @@ __device__ __forceinline__ void upd_random(R a[4], Rng<R> &rng)
     a[3] = sin_alpha * cos_theta;
 }
 
-template <int ALGO, typename R>
+// S: sites per warp of the calling layout (the heat bath runs its sites' loops on all 32 lanes, so
+// the whole warp must call it together)
+template <int ALGO, int S, typename R>
 __device__ __forceinline__ void apply_algo(R a[4], const AlgoParams &p, Rng<R> &rng)
 {
-    if (ALGO == ALG_OR) upd_or(a, p.param);
-    else if (ALGO == ALG_MICRO) upd_micro(a);
-    else if (ALGO == ALG_SA) upd_sa(a, p.param, rng);
-    else if (ALGO == ALG_SR) upd_sr(a, p.param, rng);
+    if constexpr (ALGO == ALG_OR) upd_or(a, p.param);
+    else if constexpr (ALGO == ALG_MICRO) upd_micro(a);
+    else if constexpr (ALGO == ALG_SA) upd_sa<R, S>(a, p.param, rng);
+    else if constexpr (ALGO == ALG_SR) upd_sr(a, p.param, rng);
     else upd_random(a, rng);
 }
 
@@ -439,7 +682,7 @@ __device__ __forceinline__ void subgroup_contrib(const Link<R> &up, const Link<R
 
 // From the summed quaternion to the update g (in place): MAG's factor 2 and square root, the
 // update rule, and the U1xU1 / MAG renormalisation.
-template <int GAUGE, int ALGO, typename R>
+template <int GAUGE, int ALGO, int S, typename R>
 __device__ __forceinline__ void subgroup_finish(R w[4], const AlgoParams &p, Rng<R> &rng)
 {
     if (GAUGE == MAG) {
@@ -451,7 +694,7 @@ __device__ __forceinline__ void subgroup_finish(R w[4], const AlgoParams &p, Rng
         w[1] = 0;
         w[2] = 0;
     }
-    apply_algo<ALGO>(w, p, rng);
+    apply_algo<ALGO, S>(w, p, rng);
     if (GAUGE == U1XU1) {
         w[1] = 0;
         w[2] = 0;
@@ -477,7 +720,7 @@ __device__ __forceinline__ void subgroup_step(Link<R> &up, Link<R> &dn, int mu, 
     w[1] = (GAUGE == U1XU1) ? (R)0 : site_sum(v[1]);
     w[2] = (GAUGE == U1XU1) ? (R)0 : site_sum(v[2]);
     w[3] = (GAUGE == MAG) ? (R)0 : site_sum(v[3]);
-    subgroup_finish<GAUGE, ALGO>(w, p, rng);
+    subgroup_finish<GAUGE, ALGO, 8>(w, p, rng);
     left_mult<I, J>(up, w);
     const R h[4] = {w[0], -w[1], -w[2], -w[3]};
     right_mult<I, J>(dn, h);
@@ -492,6 +735,7 @@ template <int GAUGE, int ALGO, int I, int J, typename R, bool SITE_W = false>
 __device__ __forceinline__ void subgroup_step_site(Link<R> (&up)[4], Link<R> (&dn)[4], const AlgoParams &p,
                                                    Rng<R> &rng, Cx<R> (*wcols)[2][3] = nullptr)
 {
+    static_assert(ALGO != ALG_SA, "the heat bath runs with two or four lanes per site");
     R v[4][4], w[4];
 #pragma unroll
     for (int mu = 0; mu < 4; mu++) subgroup_contrib<GAUGE, I, J>(up[mu], dn[mu], mu, v[mu]);
@@ -499,7 +743,7 @@ __device__ __forceinline__ void subgroup_step_site(Link<R> (&up)[4], Link<R> (&d
     for (int k = 0; k < 4; k++) w[k] = (v[0][k] + v[1][k]) + (v[2][k] + v[3][k]);
     if (GAUGE == U1XU1) w[1] = w[2] = 0;
     if (GAUGE == MAG) w[3] = 0;
-    subgroup_finish<GAUGE, ALGO>(w, p, rng);
+    subgroup_finish<GAUGE, ALGO, 32>(w, p, rng);
     const R h[4] = {w[0], -w[1], -w[2], -w[3]};
 #pragma unroll
     for (int mu = 0; mu < 4; mu++) {
@@ -517,11 +761,10 @@ __device__ __forceinline__ void subgroup_step_site(Link<R> (&up)[4], Link<R> (&d
 // (v0 + v1) + (v2 + v3) -- the additions of the 4-lane butterfly, in the same order -- and both
 // lanes compute the same g.  Each lane then updates its four links, and with SITE_W column `role`
 // of the site's D = W - 1, so no lane repeats another's work except the SU(2) update itself.
-template <int GAUGE, int ALGO, int I, int J, typename R, bool SITE_W>
-__device__ __forceinline__ void subgroup_step_pair(Link<R> (&up)[2], Link<R> (&dn)[2], int role, const AlgoParams &p,
-                                                   Rng<R> &rng, Cx<R> (*wcol)[3])
+template <int GAUGE, int I, int J, typename R>
+__device__ __forceinline__ void subgroup_sum_pair(const Link<R> (&up)[2], const Link<R> (&dn)[2], int role, R w[4])
 {
-    R a[4], b[4], w[4];
+    R a[4], b[4];
     subgroup_contrib<GAUGE, I, J>(up[0], dn[0], 2 * role, a);
     subgroup_contrib<GAUGE, I, J>(up[1], dn[1], 2 * role + 1, b);
 #pragma unroll
@@ -530,7 +773,11 @@ __device__ __forceinline__ void subgroup_step_pair(Link<R> (&up)[2], Link<R> (&d
         const R v = a[k] + b[k];
         w[k] = zero ? (R)0 : v + __shfl_xor_sync(0xffffffffu, v, 16);
     }
-    subgroup_finish<GAUGE, ALGO>(w, p, rng);
+}
+template <int I, int J, typename R, bool SITE_W>
+__device__ __forceinline__ void subgroup_apply_pair(Link<R> (&up)[2], Link<R> (&dn)[2], int role, const R w[4],
+                                                    Cx<R> (*wcol)[3])
+{
     const R h[4] = {w[0], -w[1], -w[2], -w[3]};
 #pragma unroll
     for (int j = 0; j < 2; j++) {
@@ -539,11 +786,49 @@ __device__ __forceinline__ void subgroup_step_pair(Link<R> (&up)[2], Link<R> (&d
     }
     if (SITE_W) left_mult_dcolumn<I, J>(*wcol, w, role);
 }
+template <int GAUGE, int ALGO, int I, int J, typename R, bool SITE_W>
+__device__ __forceinline__ void subgroup_step_pair(Link<R> (&up)[2], Link<R> (&dn)[2], int role, const AlgoParams &p,
+                                                   Rng<R> &rng, Cx<R> (*wcol)[3])
+{
+    R w[4];
+    subgroup_sum_pair<GAUGE, I, J>(up, dn, role, w);
+    subgroup_finish<GAUGE, ALGO, 16>(w, p, rng);
+    subgroup_apply_pair<I, J, R, SITE_W>(up, dn, role, w, wcol);
+}
+
+template <int I_, int J_>
+struct Pair {
+    static constexpr int I = I_, J = J_;
+};
+
+// Calls f(Pair<I, J>()) for subgroup k in the reference order (0,2), (1,2), (0,1)
+// (SU3::perSubgroup, SU3.hxx:762-771).
+template <class F>
+__device__ __forceinline__ void on_subgroup(int k, F f)
+{
+    if (k == 0) f(Pair<0, 2>());
+    else if (k == 1) f(Pair<1, 2>());
+    else f(Pair<0, 1>());
+}
+
+// The heat bath's code is larger than the rest of the update, so its three subgroup steps share one
+// copy of it in a loop that is not unrolled; only the sums and the multiplications are there three times
+// (three copies of the rejection loop made the pass wait for instructions more than for anything else).
 
 template <int GAUGE, int ALGO, typename R, bool SITE_W = false>
 __device__ __forceinline__ void site_update_pair(Link<R> (&up)[2], Link<R> (&dn)[2], int role, const AlgoParams &p,
                                                  Rng<R> &rng, Cx<R> (*wcol)[3] = nullptr)
 {
+    if constexpr (ALGO == ALG_SA) {
+#pragma unroll 1
+        for (int k = 0; k < 3; k++) {
+            R w[4];
+            on_subgroup(k, [&](auto s) { subgroup_sum_pair<GAUGE, s.I, s.J>(up, dn, role, w); });
+            subgroup_finish<GAUGE, ALGO, 16>(w, p, rng);
+            on_subgroup(k, [&](auto s) { subgroup_apply_pair<s.I, s.J, R, SITE_W>(up, dn, role, w, wcol); });
+        }
+        return;
+    }
     subgroup_step_pair<GAUGE, ALGO, 0, 2, R, SITE_W>(up, dn, role, p, rng, wcol);
     subgroup_step_pair<GAUGE, ALGO, 1, 2, R, SITE_W>(up, dn, role, p, rng, wcol);
     subgroup_step_pair<GAUGE, ALGO, 0, 1, R, SITE_W>(up, dn, role, p, rng, wcol);

@@ -237,51 +237,39 @@ int launch_pair_rp(const gf_ctx *c, const EngineDev &e, const PassArgs &a, int b
 }
 
 template <typename R, int GAUGE, int ALGO>
-int launch_pass(const gf_ctx *c, const EngineDev &e, const PassArgs &a, const gf_ctx::PassShape &sh)
+int launch_pair(const gf_ctx *c, const EngineDev &e, const PassArgs &a)
 {
-    // two lanes per site: 7 = persistent with register prefetch (OR), 6 = direct (every rule, and
-    // the other rules when 7 is chosen); Coulomb slices too (no W tracking: theirs rides in the
-    // temporal planes)
-    if constexpr (ALGO == ALG_OR && sizeof(R) == 4) {  // FP64 would spill at 255 registers
-        if (sh.variant == 7) {
-            if constexpr (GAUGE != COULOMB) {
-                if (c->site_w) {
-                    if (sh.capped) return launch_pair_rp<R, GAUGE, ALGO, true, 3>(c, e, a, sh.blocks_per_sm);
-                    return launch_pair_rp<R, GAUGE, ALGO, true>(c, e, a, sh.blocks_per_sm);
-                }
-            }
-            // capped: 168 registers, 3 blocks of 4 warps per SM instead of 2
-            if (sh.capped) return launch_pair_rp<R, GAUGE, ALGO, false, 3>(c, e, a, sh.blocks_per_sm);
-            return launch_pair_rp<R, GAUGE, ALGO, false>(c, e, a, sh.blocks_per_sm);
-        }
-    }
-    if (sh.variant == 6 || sh.variant == 7) {
-        const unsigned blocks = grid_for((a.c->total_warps + 1) / 2 * 32, 128);
-        if constexpr (sizeof(R) == 4) {
-            bool done = false;
-            if constexpr (GAUGE != COULOMB) {
-                if (c->site_w) {
-                    k_batched_pass_pair<R, GAUGE, ALGO, true, 4><<<blocks, 128, 0, a.c->stream>>>(
-                        e, a.c->total_warps, a.parity, a.p, a.want_state);
-                    done = true;
-                }
-            }
-            if (!done)
-                k_batched_pass_pair<R, GAUGE, ALGO, false, 4><<<blocks, 128, 0, a.c->stream>>>(
+    const unsigned blocks = grid_for((a.c->total_warps + 1) / 2 * 32, 128);
+    if constexpr (sizeof(R) == 4) {
+        bool done = false;
+        if constexpr (GAUGE != COULOMB) {
+            if (c->site_w) {
+                k_batched_pass_pair<R, GAUGE, ALGO, true, 4><<<blocks, 128, 0, a.c->stream>>>(
                     e, a.c->total_warps, a.parity, a.p, a.want_state);
-        } else {
-            k_batched_pass_pair<R, GAUGE, ALGO, false, 2><<<blocks, 128, 0, a.c->stream>>>(
-                e, a.c->total_warps, a.parity, a.p, a.want_state);
+                done = true;
+            }
         }
-        return launch_status("batched parity pass (two lanes per site)");
+        if (!done)
+            k_batched_pass_pair<R, GAUGE, ALGO, false, 4><<<blocks, 128, 0, a.c->stream>>>(
+                e, a.c->total_warps, a.parity, a.p, a.want_state);
+    } else {
+        k_batched_pass_pair<R, GAUGE, ALGO, false, 2><<<blocks, 128, 0, a.c->stream>>>(
+            e, a.c->total_warps, a.parity, a.p, a.want_state);
     }
+    return launch_status("batched parity pass (two lanes per site)");
+}
+
+// the shapes of four lanes and of one thread per site
+template <typename R, int GAUGE, int ALGO>
+int launch_other(const gf_ctx *c, const EngineDev &e, const PassArgs &a, const gf_ctx::PassShape &sh)
+{
     if constexpr (sizeof(R) == 4 && GAUGE != COULOMB && ALGO == ALG_OR) {
         if (sh.variant == 5) {
             if (c->site_w) return launch_site_staged<GAUGE, ALGO, true>(c, e, a, sh.blocks_per_sm);
             return launch_site_staged<GAUGE, ALGO, false>(c, e, a, sh.blocks_per_sm);
         }
     }
-    if constexpr (sizeof(R) == 4 && GAUGE != COULOMB) {
+    if constexpr (sizeof(R) == 4 && GAUGE != COULOMB && ALGO != ALG_SA) {
         if (sh.variant == 4 || sh.variant == 5) {  // one thread per site (FP32); 5 = OR-only pipelined
             const unsigned blocks = grid_for(a.c->total_warps * 8, 128);
             if (c->site_w)
@@ -333,6 +321,35 @@ int launch_pass(const gf_ctx *c, const EngineDev &e, const PassArgs &a, const gf
     k_batched_pass<R, GAUGE, ALGO><<<blocks, 128, 0, a.c->stream>>>(e, a.c->total_warps, a.parity, a.p,
                                                                      a.want_state);
     return launch_status("batched parity pass");
+}
+
+template <typename R, int GAUGE, int ALGO>
+int launch_pass(const gf_ctx *c, const EngineDev &e, const PassArgs &a, const gf_ctx::PassShape &sh)
+{
+    // two lanes per site: 7 = persistent with register prefetch (OR), 6 = direct (every rule, and
+    // the other rules when 7 is chosen); Coulomb slices too (no W tracking: theirs rides in the
+    // temporal planes)
+    if constexpr (ALGO == ALG_OR && sizeof(R) == 4) {  // FP64 would spill at 255 registers
+        if (sh.variant == 7) {
+            if constexpr (GAUGE != COULOMB) {
+                if (c->site_w) {
+                    if (sh.capped) return launch_pair_rp<R, GAUGE, ALGO, true, 3>(c, e, a, sh.blocks_per_sm);
+                    return launch_pair_rp<R, GAUGE, ALGO, true>(c, e, a, sh.blocks_per_sm);
+                }
+            }
+            // capped: 168 registers, 3 blocks of 4 warps per SM instead of 2
+            if (sh.capped) return launch_pair_rp<R, GAUGE, ALGO, false, 3>(c, e, a, sh.blocks_per_sm);
+            return launch_pair_rp<R, GAUGE, ALGO, false>(c, e, a, sh.blocks_per_sm);
+        }
+    }
+    if (sh.variant == 6 || sh.variant == 7) return launch_pair<R, GAUGE, ALGO>(c, e, a);
+    // The heat bath goes by size, whatever shape OR was tuned to.  With W tracked it stays with the
+    // tuned layout: the two layouts round W's columns differently (the links they do not).
+    if constexpr (ALGO == ALG_SA) {
+        if (!(sizeof(R) == 4 && c->site_w) && pair_fills(a.c->total_warps, c->num_sms, sizeof(R) == 8))
+            return launch_pair<R, GAUGE, ALGO>(c, e, a);
+    }
+    return launch_other<R, GAUGE, ALGO>(c, e, a, sh);
 }
 
 template <int GAUGE, int ALGO>

@@ -29,6 +29,12 @@ inline bool valid_real(int real) { return real == GF_FP32 || real == GF_FP64; }
 inline double prefactor_gff(int gauge) { return gauge == GF_COULOMB ? 1.0 / 9.0 : 1.0 / 12.0; }
 inline double prefactor_a(int) { return 1.0 / 3.0; }
 
+// Whether a pass over `tiles` 8-site tiles fills the device with two lanes per site; below that, four
+// lanes per site put twice the warps on it.  Landau heat bath, us per pass with four / two lanes: FP64
+// 8^4 (256 tiles) 10.7 / 12.7, 12^4 (1296) 18.1 / 14.7, 16^4 (4096) 33.8 / 25.2; FP32 8^4 8.9 / 10.5,
+// 12^4 10.6 / 11.2, 16^4 19.0 / 15.0.  FP64 is bound by its arithmetic pipe, so fewer warps fill it.
+inline bool pair_fills(int64_t tiles, int sms, bool fp64) { return tiles > (int64_t)sms * (fp64 ? 4 : 16); }
+
 // compile-time dispatch of a functor over the gauge / algorithm template parameters
 template <template <int, int> class K, typename... Args>
 int dispatch_gauge_algo(int gauge, int algo, const Args &...args)

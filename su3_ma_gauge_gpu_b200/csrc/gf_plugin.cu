@@ -80,6 +80,36 @@ struct StepArgs {
     cudaStream_t stream;
 };
 
+// The rules that run with two lanes per site on the reference layout (k_parity_pass_pair) where that
+// fills the device; the others always run with four.  The heat bath in both precisions, and in FP32 the
+// other rules that draw random numbers (32^4: random 80 us per pass against 110 us with four lanes, SR
+// 82 against 106; in FP64 the pass holds 246 registers and is slower, 247 against 238 us).  U1xU1's
+// stochastic and random rules stay with four lanes: there the compiler contracts the two layouts'
+// products differently, everywhere else they agree to the last bit.
+template <typename R>
+constexpr bool pair_rule(int gauge, int algo)
+{
+    return algo == ALG_SA || (sizeof(R) == 4 && (algo == ALG_SR || algo == ALG_RANDOM) && gauge != U1XU1);
+}
+
+int num_sms()
+{
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        sms = 148;
+    return sms;
+}
+
+template <typename R, int GAUGE, int ALGO>
+int launch_pair(const StepArgs &a, int64_t h_lo, int64_t h_hi, int64_t rng_site_offset)
+{
+    const RefField<R> fu{(R *)a.U, a.g.V}, fd{(R *)(a.Udw ? a.Udw : a.U), a.g.V};
+    const int64_t warps = (h_hi - (h_lo & ~(int64_t)7) + 15) / 16;
+    k_parity_pass_pair<R, GAUGE, ALGO, RefField<R>, sizeof(R) == 4 ? 4 : 2>
+        <<<(unsigned)((warps + 3) / 4), 128, 0, a.stream>>>(fu, fd, a.g, a.parity, a.p, h_lo, h_hi, rng_site_offset);
+    return launch_status("parity pass (two lanes per site)");
+}
+
 template <int GAUGE, int ALGO>
 struct RefStep {
     template <typename R>
@@ -122,6 +152,9 @@ struct RefStep {
             const unsigned blocks = (unsigned)std::max<int64_t>(1, std::min<int64_t>(need, (int64_t)sms * per_sm));
             kern<<<blocks, 128, smem, a.stream>>>(fu, fd, a.g, a.parity, a.p);
             return launch_status("parity pass (cp.async pipelined)");
+        }
+        if constexpr (pair_rule<R>(GAUGE, ALGO)) {
+            if (pair_fills(ntiles, num_sms(), sizeof(R) == 8)) return launch_pair<R, GAUGE, ALGO>(a, 0, a.g.Vh, 0);
         }
         const int64_t threads = a.g.Vh * 4;
         const unsigned blocks = (unsigned)((threads + 127) / 128);
@@ -177,9 +210,13 @@ struct RefStepRange {
             set_error("timeslice ranges are for the 4D gauges");
             return GF_ERR_INVALID;
         } else {
-            RefField<R> fu{(R *)r.a.U, r.a.g.V};
             const int64_t warps = (r.h_hi - (r.h_lo & ~(int64_t)7) + 7) / 8;
             if (warps <= 0) return GF_OK;
+            if constexpr (pair_rule<R>(GAUGE, ALGO)) {
+                if (pair_fills(warps, num_sms(), sizeof(R) == 8))
+                    return launch_pair<R, GAUGE, ALGO>(r.a, r.h_lo, r.h_hi, r.rng_site_offset);
+            }
+            RefField<R> fu{(R *)r.a.U, r.a.g.V};
             const unsigned blocks = (unsigned)((warps * 32 + 127) / 128);
             k_parity_pass_range<R, GAUGE, ALGO, RefField<R>><<<blocks, 128, 0, r.a.stream>>>(
                 fu, r.a.g, r.a.parity, r.a.p, r.h_lo, r.h_hi, r.rng_site_offset);
