@@ -1331,7 +1331,7 @@ __device__ __forceinline__ int track_progress(EngineDev e, int i, double tn)
 }
 
 template <int GAUGE, typename R, int NT = 256>
-__global__ void __launch_bounds__(NT) k_batched_quality(EngineDev e, int64_t total_blocks, CheckParams cp)
+__global__ void __launch_bounds__(NT, 2) k_batched_quality(EngineDev e, int64_t total_blocks, CheckParams cp)
 {
     const int64_t b = blockIdx.x;
     const int i = find_instance(e.inst, e.ninst, b, [](const InstDesc &d) { return d.qblock_begin; });

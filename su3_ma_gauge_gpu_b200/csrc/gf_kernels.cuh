@@ -325,37 +325,44 @@ __device__ __forceinline__ void load_link_f64(const F &f, int64_t s, int mu, Lin
     rows_f64(r, L);
 }
 
-// Visit the up link U_mu(x), then the down link U_mu(x - mu), of every direction mu >= mu0, in
-// FP64, in the order mu = mu0 .. 3 (so the arithmetic of the visitors runs in that order).  FP32
-// fields load the rows of all these links (at most 96 floats) before any arithmetic, so the eight
-// loads of a site are in flight together; FP64 fields load one link at a time.
+// Visit the up link U_mu(x), then the down link U_mu(x - mu), of every direction mu = MU0 .. 3, in FP64
+// and in that order.  The next rows are loaded before the current link's arithmetic -- the next
+// direction's two links of an FP32 field, the next link of an FP64 field, 24 registers each -- and the
+// loop is not unrolled, so no more than that is ever held and two blocks of 256 share an SM.  Bound by
+// latency (loads and the serial FP64 chain of a link), not by DRAM.  32^4: FP32 142 -> 101 us (all eight
+// links loaded at once held over 128 registers), FP64 on the reference layout 161 -> 153 us; MAG 48^4
+// FP32 723 -> 472 us.
 template <typename R, int MU0, class F, class Up, class Down>
 __device__ __forceinline__ void visit_site_links(const F &f, const Geom &g, int64_t s, const int32_t c[4], Up up,
                                                  Down down)
 {
-    if constexpr (sizeof(R) == 4) {
-        R ru[4][12], rd[4][12];
-#pragma unroll
-        for (int mu = MU0; mu < 4; mu++) {
-            f.load12(s, mu, ru[mu]);
-            f.load12(neighbour_down(g, c, mu), mu, rd[mu]);
-        }
-#pragma unroll
-        for (int mu = MU0; mu < 4; mu++) {
-            Link<double> u;
-            rows_f64(ru[mu], u);
-            up(u);
-            rows_f64(rd[mu], u);
-            down(u);
-        }
-    } else {
+    R ru[12], rd[12];
+    f.load12(s, MU0, ru);
+    if constexpr (sizeof(R) == 4) f.load12(neighbour_down(g, c, MU0), MU0, rd);
 #pragma unroll 1
-        for (int mu = MU0; mu < 4; mu++) {
-            Link<double> u;
-            load_link_f64<R>(f, s, mu, u);
-            up(u);
-            load_link_f64<R>(f, neighbour_down(g, c, mu), mu, u);
-            down(u);
+    for (int mu = MU0; mu < 4; mu++) {
+        Link<double> l;
+        if constexpr (sizeof(R) == 4) {
+            const int next = mu < 3 ? mu + 1 : mu;
+            R nu[12], nd[12];
+            f.load12(s, next, nu);
+            f.load12(neighbour_down(g, c, next), next, nd);
+            rows_f64(ru, l);
+            up(l);
+            rows_f64(rd, l);
+            down(l);
+#pragma unroll
+            for (int k = 0; k < 12; k++) {
+                ru[k] = nu[k];
+                rd[k] = nd[k];
+            }
+        } else {
+            f.load12(neighbour_down(g, c, mu), mu, rd);
+            rows_f64(ru, l);
+            up(l);
+            f.load12(s, mu < 3 ? mu + 1 : mu, ru);
+            rows_f64(rd, l);
+            down(l);
         }
     }
 }
@@ -364,6 +371,8 @@ __device__ __forceinline__ void visit_site_links(const F &f, const Geom &g, int6
 //  LANDAU/U1XU1 (LandauKernelsSU3.hxx:114-191, U1xU1KernelsSU3.hxx:114-191) and COULOMB
 //  (CoulombKernelsSU3.hxx:110-183, mu = 1..3): gff = sum_mu Re tr U_mu(x);
 //  theta = sum_ij |(A - A^dagger)_ij|^2, A = D - tr(D)/3, D = sum_mu U_mu(x) - U_mu(x-mu).
+//  A - A^dagger is antihermitian, so only its three upper off-diagonal elements and the imaginary part of
+//  its diagonal are summed: 9 numbers instead of D's 18, which is what lets two blocks share an SM.
 //  MAG (MAGKernelsSU3.hxx:116-223): gff = sum_mu sum_j |U_mu(x)_jj|^2, theta = sum_k |X_k|.
 template <int GAUGE, typename R, class F>
 __device__ __forceinline__ void quality_site(const F &f, const Geom &g, int64_t s, double &gff, double &th)
@@ -374,68 +383,64 @@ __device__ __forceinline__ void quality_site(const F &f, const Geom &g, int64_t 
     gff = 0;
     if (GAUGE == MAG) {
         double X[3][2] = {{0, 0}, {0, 0}, {0, 0}};
-        Link<double> u;
-        visit_site_links<R, 0>(f, g, s, c, [&](const Link<double> &l) { u = l; }, [&](const Link<double> &d) {
-            gff += abs2(u.e[0][0]) + abs2(u.e[1][1]) + abs2(u.e[2][2]);
+        visit_site_links<R, 0>(
+            f, g, s, c,
+            [&](const Link<double> &u) {
+                gff += abs2(u.e[0][0]) + abs2(u.e[1][1]) + abs2(u.e[2][2]);
 #pragma unroll
-            for (int k = 0; k < 3; k++) {
-                const int i = k == 2 ? 1 : 0, j = k == 0 ? 1 : 2;  // (0,1), (0,2), (1,2)
-                const Cx<double> a = u.e[i][i], b = u.e[i][j], cc = u.e[j][i], e = u.e[j][j];
-                // up: m00 conj(m10) - m01 conj(m11)
-                X[k][0] += (a.x * cc.x + a.y * cc.y) - (b.x * e.x + b.y * e.y);
-                X[k][1] += (a.y * cc.x - a.x * cc.y) - (b.y * e.x - b.x * e.y);
-                // down, hermitian submatrix: conj(d_ii) d_ij - conj(d_ji) d_jj
-                const Cx<double> p = d.e[i][i], q = d.e[i][j], r = d.e[j][i], t = d.e[j][j];
-                X[k][0] += (p.x * q.x + p.y * q.y) - (r.x * t.x + r.y * t.y);
-                X[k][1] += (p.x * q.y - p.y * q.x) - (r.x * t.y - r.y * t.x);
-            }
-        });
+                for (int k = 0; k < 3; k++) {
+                    const int i = k == 2 ? 1 : 0, j = k == 0 ? 1 : 2;  // (0,1), (0,2), (1,2)
+                    const Cx<double> a = u.e[i][i], b = u.e[i][j], cc = u.e[j][i], e = u.e[j][j];
+                    // up: m00 conj(m10) - m01 conj(m11)
+                    X[k][0] += (a.x * cc.x + a.y * cc.y) - (b.x * e.x + b.y * e.y);
+                    X[k][1] += (a.y * cc.x - a.x * cc.y) - (b.y * e.x - b.x * e.y);
+                }
+            },
+            [&](const Link<double> &d) {
+#pragma unroll
+                for (int k = 0; k < 3; k++) {
+                    const int i = k == 2 ? 1 : 0, j = k == 0 ? 1 : 2;
+                    // down, hermitian submatrix: conj(d_ii) d_ij - conj(d_ji) d_jj
+                    const Cx<double> p = d.e[i][i], q = d.e[i][j], r = d.e[j][i], t = d.e[j][j];
+                    X[k][0] += (p.x * q.x + p.y * q.y) - (r.x * t.x + r.y * t.y);
+                    X[k][1] += (p.x * q.y - p.y * q.x) - (r.x * t.y - r.y * t.x);
+                }
+            });
         th = sqrt(X[0][0] * X[0][0] + X[0][1] * X[0][1]) + sqrt(X[1][0] * X[1][0] + X[1][1] * X[1][1]) +
              sqrt(X[2][0] * X[2][0] + X[2][1] * X[2][1]);
     } else {
-        Cx<double> D[3][3];
-#pragma unroll
-        for (int i = 0; i < 3; i++)
-#pragma unroll
-            for (int j = 0; j < 3; j++) D[i][j] = cx<double>(0, 0);
+        double off[3][2] = {{0, 0}, {0, 0}, {0, 0}}, diag[3] = {0, 0, 0};
         visit_site_links<R, GAUGE == COULOMB ? 1 : 0>(
             f, g, s, c,
             [&](const Link<double> &u) {
                 gff += u.e[0][0].x + u.e[1][1].x + u.e[2][2].x;
 #pragma unroll
-                for (int i = 0; i < 3; i++)
-#pragma unroll
-                    for (int j = 0; j < 3; j++) {
-                        D[i][j].x += u.e[i][j].x;
-                        D[i][j].y += u.e[i][j].y;
-                    }
+                for (int k = 0; k < 3; k++) {
+                    const int i = k == 2 ? 1 : 0, j = k == 0 ? 1 : 2;
+                    // (D - D^dagger)_ij = D_ij - conj(D_ji)
+                    off[k][0] += u.e[i][j].x - u.e[j][i].x;
+                    off[k][1] += u.e[i][j].y + u.e[j][i].y;
+                    diag[k] += u.e[k][k].y;
+                }
             },
             [&](const Link<double> &d) {
 #pragma unroll
-                for (int i = 0; i < 3; i++)
-#pragma unroll
-                    for (int j = 0; j < 3; j++) {
-                        D[i][j].x -= d.e[i][j].x;
-                        D[i][j].y -= d.e[i][j].y;
-                    }
+                for (int k = 0; k < 3; k++) {
+                    const int i = k == 2 ? 1 : 0, j = k == 0 ? 1 : 2;
+                    off[k][0] -= d.e[i][j].x - d.e[j][i].x;
+                    off[k][1] -= d.e[i][j].y + d.e[j][i].y;
+                    diag[k] -= d.e[k][k].y;
+                }
             });
-        const double trx = (D[0][0].x + D[1][1].x + D[2][2].x) / 3.0;
-        const double try_ = (D[0][0].y + D[1][1].y + D[2][2].y) / 3.0;
+        const double tr = (diag[0] + diag[1] + diag[2]) / 3.0;
+        double acc = 0, dd = 0;
 #pragma unroll
-        for (int i = 0; i < 3; i++) {
-            D[i][i].x -= trx;
-            D[i][i].y -= try_;
+        for (int k = 0; k < 3; k++) {
+            acc += off[k][0] * off[k][0] + off[k][1] * off[k][1];
+            const double t = diag[k] - tr;
+            dd += t * t;
         }
-        double acc = 0;
-#pragma unroll
-        for (int i = 0; i < 3; i++)
-#pragma unroll
-            for (int j = 0; j < 3; j++) {
-                const double rx = D[i][j].x - D[j][i].x;  // (A - A^dagger)_ij = A_ij - conj(A_ji)
-                const double ry = D[i][j].y + D[j][i].y;
-                acc += rx * rx + ry * ry;
-            }
-        th = acc;
+        th = 2.0 * acc + 4.0 * dd;  // ij and ji; (2 Im)^2
     }
 }
 
@@ -470,7 +475,7 @@ __device__ __forceinline__ void block_reduce2(double &a, double &b, bool b_is_ma
 }
 
 struct QualityOut {
-    double *partials;    // 2 doubles per block
+    double *partials;    // 2 doubles per block, or null: per-site values only
     unsigned int *ticket; // zero before the launch; the last block resets it
     double *result;      // [0] = functional, [1] = theta (normalised as the reference does)
     double *gff_site;    // optional per-site arrays (generateGaugeQualityPerSite), may be null
@@ -480,8 +485,9 @@ struct QualityOut {
 // GaugeFixingStats::generateGaugeQuality (GaugeFixingStats.hxx:186-232) in one launch: per-site
 // values, per-block partial sums, and the last block to finish sums the partials in block
 // order and applies the normalisation gff*preG/V, theta*preA (/V for AVERAGE).
+// With o.partials null only the per-site arrays are written.
 template <int GAUGE, typename R, class F, int NT = 256>
-__global__ void __launch_bounds__(NT) k_quality(F f, Geom g, QualityOut o, int stop_max, double preG, double preA)
+__global__ void __launch_bounds__(NT, 2) k_quality(F f, Geom g, QualityOut o, int stop_max, double preG, double preA)
 {
     const int64_t s = (int64_t)blockIdx.x * NT + threadIdx.x;
     double gv = 0, tv = 0;
@@ -490,6 +496,7 @@ __global__ void __launch_bounds__(NT) k_quality(F f, Geom g, QualityOut o, int s
         if (o.gff_site) o.gff_site[s] = gv;
         if (o.theta_site) o.theta_site[s] = tv;
     }
+    if (!o.partials) return;
     block_reduce2<NT>(gv, tv, stop_max != 0);
     __shared__ bool last;
     if (threadIdx.x == 0) {

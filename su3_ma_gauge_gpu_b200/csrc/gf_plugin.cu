@@ -445,24 +445,25 @@ int gf_stats_destroy(gf_stats *s)
 int gf_quality_per_site(int gauge, int real, const void *U, const int32_t size[4], double *dGff, double *dA,
                         void *stream)
 {
-    gf_stats *s = nullptr;
-    int st = gf_stats_create(gauge, real, size, GF_AVERAGE, &s);
-    if (st) return st;
+    clear_error();
+    if (!valid_gauge(gauge) || !valid_real(real)) {
+        set_error("invalid argument to gf_quality_per_site");
+        return GF_ERR_INVALID;
+    }
     QualityArgs a;
+    int st = make_geom(size, gauge, true, a.g);
+    if (st) return st;
+    if (!U) {
+        set_error("field is NULL");
+        return GF_ERR_INVALID;
+    }
     a.real = real;
     a.U = U;
-    a.g = s->g;
-    a.o.partials = s->scratch;
-    a.o.result = s->scratch + 2 * (size_t)s->blocks;
-    a.o.ticket = s->ticket;
-    a.o.gff_site = dGff;
-    a.o.theta_site = dA;
+    a.o = QualityOut{nullptr, nullptr, nullptr, dGff, dA};  // no reduction, so nothing to allocate
     a.stop_max = 0;
     a.stream = (cudaStream_t)stream;
-    st = U ? quality_dispatch(gauge, a) : (set_error("field is NULL"), GF_ERR_INVALID);
-    if (!st) st = cuda_status(cudaStreamSynchronize(a.stream), "cudaStreamSynchronize");
-    gf_stats_destroy(s);
-    return st;
+    if ((st = quality_dispatch(gauge, a))) return st;
+    return cuda_status(cudaStreamSynchronize(a.stream), "cudaStreamSynchronize");
 }
 
 int gf_project_su3(int real, void *U, const int32_t size[4], void *stream)
