@@ -854,6 +854,138 @@ __device__ __forceinline__ void site_update_thread(Link<R> (&up)[4], Link<R> (&d
     subgroup_step_site<GAUGE, ALGO, 0, 1, R, SITE_W>(up, dn, p, rng, wcols);
 }
 
+// ---- two links at a time in packed FP32 arithmetic -------------------------------------------------
+// The persistent FP32 passes with two lanes per site are bound by instruction issue (63 % of the issue
+// slots, 1632 instructions per 16-site tile), and the multiplications of a lane's two up links, and
+// of its two down links, by the same SU(2) element are the same instructions on different data.  Here
+// the two links share float2 registers and every multiply and add of them is one packed instruction
+// (FMUL2 / FFMA2 / FADD2): 39 M instructions per 32^4 pass instead of 53 M.  us per pass, scalar /
+// packed: Coulomb 16 slices of 48^3 116.8 / 104.9, Landau 32^4 in FP32 storage 68.4 / 66.6 (6.05 TB/s).
+// With W tracked (refine mode) it gains nothing, 79.8 / 79.3 (MAG 48^4 393 / 415): there the register
+// cap that buys 12 warps per SM leaves no room for the pairs, so that pass stays scalar.
+// The products are added in the order the compiler gives the scalar functions
+// above, (fma, product) + (fma, product), so the results are those of the other passes to the last bit.
+struct Link2 {
+    float2 x[3][3], y[3][3];  // .x: the link of direction 2 role, .y: that of 2 role + 1
+};
+__device__ __forceinline__ float2 both(float v) { return make_float2(v, v); }
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+__device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
+// (a b + c d) + (e f + g h), each product pair as one fma on a rounded product
+__device__ __forceinline__ float2 two_pairs(float2 a, float2 b, float2 c, float2 d, float2 e, float2 f, float2 g, float2 h)
+{
+    return add2(fma2(a, b, mul2(c, d)), fma2(e, f, mul2(g, h)));
+}
+
+__device__ __forceinline__ void pack_rows(Link2 &L, const float a[12], const float b[12])
+{
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+#pragma unroll
+        for (int j = 0; j < 3; j++) {
+            L.x[i][j] = make_float2(a[2 * (3 * i + j)], b[2 * (3 * i + j)]);
+            L.y[i][j] = make_float2(a[2 * (3 * i + j) + 1], b[2 * (3 * i + j) + 1]);
+        }
+}
+// the rows of one of the two links (half = 0, 1)
+__device__ __forceinline__ void unpack_rows(const Link2 &L, int half, float r[12])
+{
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+#pragma unroll
+        for (int j = 0; j < 3; j++) {
+            r[2 * (3 * i + j)] = half ? L.x[i][j].y : L.x[i][j].x;
+            r[2 * (3 * i + j) + 1] = half ? L.y[i][j].y : L.y[i][j].x;
+        }
+}
+__device__ __forceinline__ void one_of(const Link2 &L, int half, Link<float> &o)
+{
+#pragma unroll
+    for (int i = 0; i < 3; i++)
+#pragma unroll
+        for (int j = 0; j < 3; j++)
+            o.e[i][j] = half ? cx<float>(L.x[i][j].y, L.y[i][j].y) : cx<float>(L.x[i][j].x, L.y[i][j].x);
+}
+
+// reconstruct() of both links
+__device__ __forceinline__ void reconstruct2(Link2 &L)
+{
+    const float2 minus = both(-1.f);
+    float2 nx[3], ny[3], cx_[3], cy_[3];  // -row1; the cross product
+#pragma unroll
+    for (int j = 0; j < 3; j++) {
+        nx[j] = mul2(L.x[1][j], minus);
+        ny[j] = mul2(L.y[1][j], minus);
+    }
+#pragma unroll
+    for (int j = 0; j < 3; j++) {
+        const int p = (j + 1) % 3, q = (j + 2) % 3;
+        cx_[j] = two_pairs(L.x[0][p], L.x[1][q], L.y[0][p], ny[q], L.x[0][q], nx[p], L.y[0][q], L.y[1][p]);
+        cy_[j] = two_pairs(L.y[0][p], nx[q], L.x[0][p], ny[q], L.y[0][q], L.x[1][p], L.x[0][q], L.y[1][p]);
+    }
+    float2 n[3];
+#pragma unroll
+    for (int j = 0; j < 3; j++) n[j] = fma2(cx_[j], cx_[j], mul2(cy_[j], cy_[j]));
+    const float2 sum = add2(add2(n[0], n[1]), n[2]);
+    const float2 inv = make_float2(rsq(sum.x), rsq(sum.y));
+#pragma unroll
+    for (int j = 0; j < 3; j++) {
+        L.x[2][j] = mul2(cx_[j], inv);
+        L.y[2][j] = mul2(cy_[j], inv);
+    }
+}
+
+// left_mult<I, J>(up, g) and right_mult<I, J>(dn, g^dagger) of two links each
+template <int I, int J>
+__device__ __forceinline__ void subgroup_mult2(Link2 &up, Link2 &dn, const float g[4])
+{
+    const float2 g0 = both(g[0]), g1 = both(g[1]), g2 = both(g[2]), g3 = both(g[3]);
+    const float2 n1 = both(-g[1]), n2 = both(-g[2]), n3 = both(-g[3]);
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        const float2 ax = up.x[I][k], ay = up.y[I][k], bx = up.x[J][k], by = up.y[J][k];
+        up.x[I][k] = two_pairs(g0, ax, n3, ay, g2, bx, n1, by);
+        up.y[I][k] = two_pairs(g3, ax, g0, ay, g1, bx, g2, by);
+        up.x[J][k] = two_pairs(n2, ax, n1, ay, g0, bx, g3, by);
+        up.y[J][k] = two_pairs(g1, ax, n2, ay, g0, by, n3, bx);
+    }
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        const float2 ax = dn.x[k][I], ay = dn.y[k][I], bx = dn.x[k][J], by = dn.y[k][J];
+        dn.x[k][I] = two_pairs(g0, ax, g3, ay, g2, bx, g1, by);
+        dn.y[k][I] = two_pairs(g0, ay, n3, ax, g2, by, n1, bx);
+        dn.x[k][J] = two_pairs(g1, ay, n2, ax, g0, bx, n3, by);
+        dn.y[k][J] = two_pairs(n1, ax, n2, ay, g3, bx, g0, by);
+    }
+}
+
+template <int GAUGE, int ALGO, int I, int J>
+__device__ __forceinline__ void subgroup_step_pair2(Link2 &up, Link2 &dn, int role, const AlgoParams &p, Rng<float> &rng)
+{
+    Link<float> u[2], d[2];
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        one_of(up, h, u[h]);
+        one_of(dn, h, d[h]);
+    }
+    float w[4];
+    subgroup_sum_pair<GAUGE, I, J>(u, d, role, w);
+    subgroup_finish<GAUGE, ALGO, 16>(w, p, rng);
+    subgroup_mult2<I, J>(up, dn, w);
+}
+
+// site_update_pair for the rules that draw no random numbers, without W
+template <int GAUGE, int ALGO>
+__device__ __forceinline__ void site_update_pair2(Link2 &up, Link2 &dn, int role, const AlgoParams &p)
+{
+    static_assert(ALGO == ALG_OR || ALGO == ALG_MICRO, "rules without random numbers");
+    Rng<float> rng;
+    subgroup_step_pair2<GAUGE, ALGO, 0, 2>(up, dn, role, p, rng);
+    subgroup_step_pair2<GAUGE, ALGO, 1, 2>(up, dn, role, p, rng);
+    subgroup_step_pair2<GAUGE, ALGO, 0, 1>(up, dn, role, p, rng);
+}
+
 // ---- lattice geometry -----------------------------------------------------------------------
 // Division by a lattice extent without a divide instruction: for 0 <= n < 2^31 and d >= 1,
 // q = (umulhi(n, m) + n) >> s with s = ceil(log2 d), m = floor(2^32 (2^s - d) / d) + 1

@@ -142,6 +142,13 @@ constexpr int QNT = 256;
 
 unsigned grid_for(int64_t threads, int block) { return (unsigned)((threads + block - 1) / block); }
 
+// grid of the link-wise and check kernels, which walk their links: at most `per_sm` blocks per SM
+unsigned walk_grid(const gf_ctx *c, int64_t blocks, int per_sm)
+{
+    return (unsigned)std::max<int64_t>(1, std::min<int64_t>(blocks, (int64_t)c->num_sms * per_sm));
+}
+unsigned link_grid(const gf_ctx *c) { return walk_grid(c, (c->total_links + 255) / 256, 8); }
+
 // ---- batched kernel dispatch -------------------------------------------------------------------
 struct PassArgs {
     const gf_ctx *c;
@@ -216,10 +223,12 @@ int launch_site_staged(const gf_ctx *c, const EngineDev &e, const PassArgs &a, i
     return launch_status("batched parity pass (thread per site, pipelined)");
 }
 
-template <typename R, int GAUGE, int ALGO, bool SITE_W, int MINB = 1>
+template <int GAUGE, int ALGO, bool SITE_W, int MINB = 1>
 int launch_pair_rp(const gf_ctx *c, const EngineDev &e, const PassArgs &a, int blocks_per_sm)
 {
-    auto kern = k_batched_pass_pair_rp<R, GAUGE, ALGO, SITE_W, MINB>;
+    void (*kern)(EngineDev, int64_t, int, AlgoParams, int, int);
+    if constexpr (SITE_W) kern = k_batched_pass_pair_rp<float, GAUGE, ALGO, true, MINB>;
+    else kern = k_batched_pass_pair_packed<GAUGE, ALGO, MINB>;
     static int occ_cached = 0;  // resident blocks per SM of this instantiation
     int occ = blocks_per_sm;
     if (occ <= 0) {
@@ -326,20 +335,20 @@ int launch_other(const gf_ctx *c, const EngineDev &e, const PassArgs &a, const g
 template <typename R, int GAUGE, int ALGO>
 int launch_pass(const gf_ctx *c, const EngineDev &e, const PassArgs &a, const gf_ctx::PassShape &sh)
 {
-    // two lanes per site: 7 = persistent with register prefetch (OR), 6 = direct (every rule, and
-    // the other rules when 7 is chosen); Coulomb slices too (no W tracking: theirs rides in the
+    // two lanes per site: 7 = persistent with register prefetch (OR and micro), 6 = direct (every rule,
+    // and the other rules when 7 is chosen); Coulomb slices too (no W tracking: theirs rides in the
     // temporal planes)
-    if constexpr (ALGO == ALG_OR && sizeof(R) == 4) {  // FP64 would spill at 255 registers
+    if constexpr ((ALGO == ALG_OR || ALGO == ALG_MICRO) && sizeof(R) == 4) {  // FP64 would spill at 255 registers
         if (sh.variant == 7) {
             if constexpr (GAUGE != COULOMB) {
                 if (c->site_w) {
-                    if (sh.capped) return launch_pair_rp<R, GAUGE, ALGO, true, 3>(c, e, a, sh.blocks_per_sm);
-                    return launch_pair_rp<R, GAUGE, ALGO, true>(c, e, a, sh.blocks_per_sm);
+                    if (sh.capped) return launch_pair_rp<GAUGE, ALGO, true, 3>(c, e, a, sh.blocks_per_sm);
+                    return launch_pair_rp<GAUGE, ALGO, true>(c, e, a, sh.blocks_per_sm);
                 }
             }
             // capped: 168 registers, 3 blocks of 4 warps per SM instead of 2
-            if (sh.capped) return launch_pair_rp<R, GAUGE, ALGO, false, 3>(c, e, a, sh.blocks_per_sm);
-            return launch_pair_rp<R, GAUGE, ALGO, false>(c, e, a, sh.blocks_per_sm);
+            if (sh.capped) return launch_pair_rp<GAUGE, ALGO, false, 3>(c, e, a, sh.blocks_per_sm);
+            return launch_pair_rp<GAUGE, ALGO, false>(c, e, a, sh.blocks_per_sm);
         }
     }
     if (sh.variant == 6 || sh.variant == 7) return launch_pair<R, GAUGE, ALGO>(c, e, a);
@@ -383,13 +392,15 @@ int launch_sweep(const gf_ctx *c, int algo, int want_state, float param, uint32_
 
 int launch_quality(const gf_ctx *c, const CheckParams &cp)
 {
-    const unsigned blocks = (unsigned)c->total_qblocks;
+    const unsigned blocks = (unsigned)c->total_qblocks, walk = walk_grid(c, c->total_qblocks, 2);
     const EngineDev e = c->dev();
 #define GFB_Q(G)                                                                                  \
     if (cp.want_state == ST_FP32)                                                                 \
-        k_batched_quality<G, float, QNT><<<blocks, QNT, 0, c->stream>>>(e, c->total_qblocks, cp);  \
+        k_batched_quality<G, float, QNT><<<blocks, QNT, 0, c->stream>>>(e, cp);                   \
+    else if (cp.want_state == ST_FOLD)                                                            \
+        k_fold_quality<G, QNT><<<walk, QNT, 0, c->stream>>>(e, c->total_qblocks, cp);             \
     else                                                                                          \
-        k_batched_quality<G, double, QNT><<<blocks, QNT, 0, c->stream>>>(e, c->total_qblocks, cp);
+        k_batched_quality<G, double, QNT><<<blocks, QNT, 0, c->stream>>>(e, cp);
     switch (c->gauge) {
     case LANDAU: GFB_Q(LANDAU) break;
     case MAG: GFB_Q(MAG) break;
@@ -403,7 +414,7 @@ int launch_quality(const gf_ctx *c, const CheckParams &cp)
 
 int launch_reunitarise(const gf_ctx *c, int want_state, bool to64)
 {
-    const unsigned blocks = grid_for(c->total_links, 256);
+    const unsigned blocks = link_grid(c);
     if (c->refine && to64) {
         // refine switch: the FP64 master takes the accumulated W (an exact gauge transformation)
         if (c->site_w) k_apply_w<<<blocks, 256, 0, c->stream>>>(c->dev(), c->total_links);
@@ -542,7 +553,7 @@ int enqueue_or_chunk(gf_ctx *c, int nsweeps, float omega, const std::vector<unsi
         if (c->refine && cp.fold) {
             // iterative refinement: instances now in ST_FOLD fold W into the FP64 master, restart
             // the working copy, and are checked on the master (their sweeps are already counted)
-            const unsigned blocks = grid_for(c->total_links, 256);
+            const unsigned blocks = link_grid(c);
             if (c->site_w) {
                 k_reunitarise_w<<<blocks, 256, 0, c->stream>>>(c->dev(), c->total_links, ST_FOLD);
                 k_fold_apply<<<blocks, 256, 0, c->stream>>>(c->dev(), c->total_links);
@@ -1467,7 +1478,7 @@ int gf_autotune(gf_ctx *c, int *choice_fp32, int *choice_fp64)
 // `warps` = 2, 4 or 8 warps per block), 2 (FP32 direct capped at 64 registers), 3 (register
 // prefetch, persistent), 4 (FP32, one thread per site), 5 (the same, pipelined with cp.async;
 // OR only, other update rules fall back to variant 4), 6 (two lanes per site) or 7 (two lanes per
-// site, persistent with register prefetch; FP32 OR only, the other cases run as 6).
+// site, persistent with register prefetch; FP32 OR and micro, the other cases run as 6).
 int gf_set_pass_shape(gf_ctx *c, int real, int variant, int warps)
 {
     clear_error();

@@ -66,6 +66,17 @@ __device__ __forceinline__ int find_instance(const InstDesc *inst, int n, int64_
     return lo;
 }
 
+// Whether any instance is in state want; the whole block must call it.  The check and fold kernels
+// of a chunk run whether or not an instance needs them, so they are launched with a grid of a few
+// blocks per SM that walks the links, and leave here when there is nothing to do: an idle launch over
+// a 32^4 lattice costs about 2 us instead of 6 (quality) to 18 us (16384 blocks that each find out).
+__device__ __forceinline__ bool any_in_state(const EngineDev &e, int want)
+{
+    int any = 0;
+    for (int i = threadIdx.x; i < e.ninst; i += blockDim.x) any |= e.state[i] == want;
+    return __syncthreads_or(any) != 0;
+}
+
 template <typename R>
 __device__ __forceinline__ PackedField<R> packed_of(const InstDesc &d);
 template <>
@@ -469,6 +480,7 @@ __device__ __forceinline__ void fetch_pair_regs(const EngineDev &e, const InstCa
     }
 }
 
+// With W tracked (SITE_W); the passes without it run k_batched_pass_pair_packed.
 template <typename R, int GAUGE, int ALGO, bool SITE_W, int MINB = 1>
 __global__ void __launch_bounds__(128, MINB) k_batched_pass_pair_rp(EngineDev e, int64_t total_tiles, int parity,
                                                               AlgoParams p, int want_state, int reverse)
@@ -559,6 +571,59 @@ __global__ void __launch_bounds__(128, MINB) k_batched_pass_pair_rp(EngineDev e,
     if (SITE_W) cp_async_wait<0>();
 }
 
+// The same pass in packed arithmetic, two links per float2 (see Link2), for FP32 fields without the
+// separate W array: FP32 storage, and Coulomb slices, whose W rides in the temporal planes.
+template <int GAUGE, int ALGO, int MINB = 1>
+__global__ void __launch_bounds__(128, MINB) k_batched_pass_pair_packed(EngineDev e, int64_t total_tiles, int parity,
+                                                                  AlgoParams p, int want_state, int reverse)
+{
+    __shared__ InstCache ic;
+    fill_inst_cache(e, ic);
+    const int lane = threadIdx.x & 31, role = lane >> 4, half = (lane >> 3) & 1;
+    const bool wlane = GAUGE == COULOMB && role == 0;  // its direction 0 is the slice's W
+    const int64_t npair = (total_tiles + 1) / 2;                 // 16-site pair tiles
+    const int64_t stride = (int64_t)gridDim.x * 4;
+    int64_t pt = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);   // this warp's pair tile
+    PairRegs<float> cur;
+    cur.ps.inst = -1;
+    if (pt < npair)
+        fetch_pair_regs<float, GAUGE, false>(e, ic, ordered_tile(pt, npair, reverse) * 2 + half, total_tiles, parity,
+                                             want_state, cur, nullptr);
+    // every lane of a warp runs the same iterations (pt is warp-uniform), so the shuffles are safe
+    for (; pt < npair; pt += stride) {
+        PairRegs<float> nxt;
+        nxt.ps.inst = -1;
+        if (pt + stride < npair)
+            fetch_pair_regs<float, GAUGE, false>(e, ic, ordered_tile(pt + stride, npair, reverse) * 2 + half,
+                                                 total_tiles, parity, want_state, nxt, nullptr);
+        const int i = cur.ps.inst;
+        if (__any_sync(0xffffffffu, i >= 0)) {
+            // an idle tile's lanes hold no links (they exchange only with each other and store nothing),
+            // and a W lane's direction 0 no down link
+            Link2 up, dn;
+            pack_rows(up, cur.up[0], cur.up[1]);
+            pack_rows(dn, cur.dn[0], cur.dn[1]);
+            reconstruct2(up);
+            reconstruct2(dn);
+            site_update_pair2<GAUGE, ALGO>(up, dn, role, p);
+            if (i >= 0) {
+                const PackedField<float> f = packed_of<float>(inst_at(e, ic, i));
+#pragma unroll
+                for (int j = 0; j < 2; j++) {
+                    float r[12];
+                    unpack_rows(up, j, r);
+                    f.store12(cur.ps.s, 2 * role + j, r);
+                    if (!(wlane && j == 0)) {
+                        unpack_rows(dn, j, r);
+                        f.store12(cur.ps.sd[j], 2 * role + j, r);
+                    }
+                }
+            }
+        }
+        cur = nxt;
+    }
+}
+
 // ---- refine mode: FP64 master + FP32 working copy + accumulated W --------------------------------
 // W(x) is kept as the first two columns of D = W - 1 (6 float2 planes of V): storing the
 // deviation from the identity keeps FP32 relative accuracy on the small rotations of the late
@@ -625,17 +690,19 @@ __global__ void __launch_bounds__(256) k_import_refine(EngineDev e, int i, const
 // reunitarise W (FP64 arithmetic) of every instance in state want_state
 __global__ void __launch_bounds__(256) k_reunitarise_w(EngineDev e, int64_t total_links, int want_state)
 {
-    const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= total_links) return;
-    const int i = find_instance(e.inst, e.ninst, idx, [](const InstDesc &d) { return d.link_begin; });
-    if (e.state[i] != want_state) return;
-    const InstDesc d = e.inst[i];
-    const int64_t l = idx - d.link_begin;
-    if (l >= d.g.V) return;  // one thread per site: the first quarter of the instance's links
-    Link<double> W;
-    load_w_f64(d, l, W);
-    project_rows(W);
-    store_w(d, l, W);
+    if (!any_in_state(e, want_state)) return;
+    for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total_links;
+         idx += (int64_t)gridDim.x * blockDim.x) {
+        const int i = find_instance(e.inst, e.ninst, idx, [](const InstDesc &d) { return d.link_begin; });
+        if (e.state[i] != want_state) continue;
+        const InstDesc d = e.inst[i];
+        const int64_t l = idx - d.link_begin;
+        if (l >= d.g.V) continue;  // one thread per site: the first quarter of the instance's links
+        Link<double> W;
+        load_w_f64(d, l, W);
+        project_rows(W);
+        store_w(d, l, W);
+    }
 }
 
 // U64_mu(x) <- W(x) U64_mu(x) W(x+mu)^dagger, reunitarised, in FP64 (W reunitarised first unless
@@ -689,19 +756,21 @@ __device__ __forceinline__ void apply_w_link(const InstDesc &d, int64_t s, int m
 // refine switch: the FP64 master of every instance in ST_SWITCH becomes W U64 W^dagger
 __global__ void __launch_bounds__(256) k_apply_w(EngineDev e, int64_t total_links)
 {
-    const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= total_links) return;
-    const int i = find_instance(e.inst, e.ninst, idx, [](const InstDesc &d) { return d.link_begin; });
-    if (e.state[i] != ST_SWITCH) return;
-    const InstDesc d = e.inst[i];
-    const int64_t l = idx - d.link_begin;
-    const int mu = (int)(l / d.g.V);
-    const int64_t s = l - mu * d.g.V;
-    Link<double> L;
-    apply_w_link(d, s, mu, L);
-    double r[12];
-    pack12(L, r);
-    packed_of<double>(d).store12(s, mu, r);  // each thread reads and writes only its own link
+    if (!any_in_state(e, ST_SWITCH)) return;
+    for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total_links;
+         idx += (int64_t)gridDim.x * blockDim.x) {
+        const int i = find_instance(e.inst, e.ninst, idx, [](const InstDesc &d) { return d.link_begin; });
+        if (e.state[i] != ST_SWITCH) continue;
+        const InstDesc d = e.inst[i];
+        const int64_t l = idx - d.link_begin;
+        const int mu = (int)(l / d.g.V);
+        const int64_t s = l - mu * d.g.V;
+        Link<double> L;
+        apply_w_link(d, s, mu, L);
+        double r[12];
+        pack12(L, r);
+        packed_of<double>(d).store12(s, mu, r);  // each thread reads and writes only its own link
+    }
 }
 
 // iterative refinement (refine contexts, fold mode): every instance in ST_FOLD folds its
@@ -711,38 +780,42 @@ __global__ void __launch_bounds__(256) k_apply_w(EngineDev e, int64_t total_link
 // launch, because this one reads W(x + mu) of neighbouring sites.
 __global__ void __launch_bounds__(256) k_fold_apply(EngineDev e, int64_t total_links)
 {
-    const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= total_links) return;
-    const int i = find_instance(e.inst, e.ninst, idx, [](const InstDesc &d) { return d.link_begin; });
-    if (e.state[i] != ST_FOLD) return;
-    const InstDesc d = e.inst[i];
-    const int64_t l = idx - d.link_begin;
-    const int mu = (int)(l / d.g.V);
-    const int64_t s = l - mu * d.g.V;
-    Link<double> L;
-    apply_w_link(d, s, mu, L, false);  // k_reunitarise_w has projected every W of the instance
-    double r[12];
-    float f[12];
-    pack12(L, r);
+    if (!any_in_state(e, ST_FOLD)) return;
+    for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total_links;
+         idx += (int64_t)gridDim.x * blockDim.x) {
+        const int i = find_instance(e.inst, e.ninst, idx, [](const InstDesc &d) { return d.link_begin; });
+        if (e.state[i] != ST_FOLD) continue;
+        const InstDesc d = e.inst[i];
+        const int64_t l = idx - d.link_begin;
+        const int mu = (int)(l / d.g.V);
+        const int64_t s = l - mu * d.g.V;
+        Link<double> L;
+        apply_w_link(d, s, mu, L, false);  // k_reunitarise_w has projected every W of the instance
+        double r[12];
+        float f[12];
+        pack12(L, r);
 #pragma unroll
-    for (int k = 0; k < 12; k++) f[k] = (float)r[k];
-    packed_of<double>(d).store12(s, mu, r);
-    packed_of<float>(d).store12(s, mu, f);
+        for (int k = 0; k < 12; k++) f[k] = (float)r[k];
+        packed_of<double>(d).store12(s, mu, r);
+        packed_of<float>(d).store12(s, mu, f);
+    }
 }
 
 __global__ void __launch_bounds__(256) k_fold_reset_w(EngineDev e, int64_t total_links)
 {
-    const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= total_links) return;
-    const int i = find_instance(e.inst, e.ninst, idx, [](const InstDesc &d) { return d.link_begin; });
-    if (e.state[i] != ST_FOLD) return;
-    const InstDesc d = e.inst[i];
-    const int64_t l = idx - d.link_begin;
-    if (l >= d.g.V) return;  // one thread per site
+    if (!any_in_state(e, ST_FOLD)) return;
+    for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total_links;
+         idx += (int64_t)gridDim.x * blockDim.x) {
+        const int i = find_instance(e.inst, e.ninst, idx, [](const InstDesc &d) { return d.link_begin; });
+        if (e.state[i] != ST_FOLD) continue;
+        const InstDesc d = e.inst[i];
+        const int64_t l = idx - d.link_begin;
+        if (l >= d.g.V) continue;  // one thread per site
 #pragma unroll
-    for (int k = 0; k < 2; k++)
+        for (int k = 0; k < 2; k++)
 #pragma unroll
-        for (int r = 0; r < 3; r++) d.w[(int64_t)(k * 3 + r) * d.g.V + l] = make_float2(0.f, 0.f);  // D = 0
+            for (int r = 0; r < 3; r++) d.w[(int64_t)(k * 3 + r) * d.g.V + l] = make_float2(0.f, 0.f);  // D = 0
+    }
 }
 
 // export of a refine instance still in FP32: W U64 W^dagger on the fly
@@ -837,48 +910,52 @@ __device__ __forceinline__ void coulomb_apply_w32(const InstDesc &d, int64_t s, 
 template <bool FOLD>
 __global__ void __launch_bounds__(256) k_apply_w_coulomb(EngineDev e, int64_t total_links)
 {
-    const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= total_links) return;
-    const int i = find_instance(e.inst, e.ninst, idx, [](const InstDesc &d) { return d.link_begin; });
-    if (e.state[i] != (FOLD ? ST_FOLD : ST_SWITCH)) return;
-    const InstDesc d = e.inst[i];
-    const int64_t l = idx - d.link_begin;
-    const int mu = (int)(l / d.g.V);
-    const int64_t s = l - mu * d.g.V;
-    Link<double> L;
-    if (mu == 0) {
-        Link<double> W, W64;
-        coulomb_w32(d, s, W);
-        load_link_f64<double>(packed_of<double>(d), s, 0, W64);
-        mul33(W, W64, L);
-        project_rows(L);
-    } else {
-        coulomb_apply_w32(d, s, mu, L);
-    }
-    double r[12];
-    pack12(L, r);
-    packed_of<double>(d).store12(s, mu, r);  // each thread reads and writes only its own master link
-    if (FOLD && mu != 0) {
-        float f[12];
+    if (!any_in_state(e, FOLD ? ST_FOLD : ST_SWITCH)) return;
+    for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total_links;
+         idx += (int64_t)gridDim.x * blockDim.x) {
+        const int i = find_instance(e.inst, e.ninst, idx, [](const InstDesc &d) { return d.link_begin; });
+        if (e.state[i] != (FOLD ? ST_FOLD : ST_SWITCH)) continue;
+        const InstDesc d = e.inst[i];
+        const int64_t l = idx - d.link_begin;
+        const int mu = (int)(l / d.g.V);
+        const int64_t s = l - mu * d.g.V;
+        Link<double> L;
+        if (mu == 0) {
+            Link<double> W, W64;
+            coulomb_w32(d, s, W);
+            load_link_f64<double>(packed_of<double>(d), s, 0, W64);
+            mul33(W, W64, L);
+            project_rows(L);
+        } else {
+            coulomb_apply_w32(d, s, mu, L);
+        }
+        double r[12];
+        pack12(L, r);
+        packed_of<double>(d).store12(s, mu, r);  // each thread reads and writes only its own master link
+        if (FOLD && mu != 0) {
+            float f[12];
 #pragma unroll
-        for (int k = 0; k < 12; k++) f[k] = (float)r[k];
-        packed_of<float>(d).store12(s, mu, f);
+            for (int k = 0; k < 12; k++) f[k] = (float)r[k];
+            packed_of<float>(d).store12(s, mu, f);
+        }
     }
 }
 
 __global__ void __launch_bounds__(256) k_fold_coulomb_reset(EngineDev e, int64_t total_links)
 {
-    const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= total_links) return;
-    const int i = find_instance(e.inst, e.ninst, idx, [](const InstDesc &d) { return d.link_begin; });
-    if (e.state[i] != ST_FOLD) return;
-    const InstDesc d = e.inst[i];
-    const int64_t l = idx - d.link_begin;
-    if (l >= d.g.V) return;  // one thread per site: the mu = 0 planes
-    float one[12];
+    if (!any_in_state(e, ST_FOLD)) return;
+    for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total_links;
+         idx += (int64_t)gridDim.x * blockDim.x) {
+        const int i = find_instance(e.inst, e.ninst, idx, [](const InstDesc &d) { return d.link_begin; });
+        if (e.state[i] != ST_FOLD) continue;
+        const InstDesc d = e.inst[i];
+        const int64_t l = idx - d.link_begin;
+        if (l >= d.g.V) continue;  // one thread per site: the mu = 0 planes
+        float one[12];
 #pragma unroll
-    for (int k = 0; k < 12; k++) one[k] = (k == 0 || k == 8) ? 1.f : 0.f;  // rows 0,1 of 1
-    packed_of<float>(d).store12(l, 0, one);
+        for (int k = 0; k < 12; k++) one[k] = (k == 0 || k == 8) ? 1.f : 0.f;  // rows 0,1 of 1
+        packed_of<float>(d).store12(l, 0, one);
+    }
 }
 
 // ---- software-pipelined parity pass --------------------------------------------------------------
@@ -1330,10 +1407,10 @@ __device__ __forceinline__ int track_progress(EngineDev e, int i, double tn)
     return stall;
 }
 
-template <int GAUGE, typename R, int NT = 256>
-__global__ void __launch_bounds__(NT, 2) k_batched_quality(EngineDev e, int64_t total_blocks, CheckParams cp)
+template <int GAUGE, typename R, int NT>
+__device__ __forceinline__ void quality_block(const EngineDev &e, int64_t b, const CheckParams &cp)
 {
-    const int64_t b = blockIdx.x;
+    __shared__ bool last;
     const int i = find_instance(e.inst, e.ninst, b, [](const InstDesc &d) { return d.qblock_begin; });
     // with transitions: the instances sweeping in this precision; without: every instance whose
     // field lives in this precision (uniform over the block)
@@ -1344,7 +1421,6 @@ __global__ void __launch_bounds__(NT, 2) k_batched_quality(EngineDev e, int64_t 
     double gv = 0, tv = 0;
     if (s < d.g.V) quality_site<GAUGE, R>(packed_of<R>(d), d.g, s, gv, tv);
     block_reduce2<NT>(gv, tv, cp.stop_max != 0);
-    __shared__ bool last;
     if (threadIdx.x == 0) {
         e.partials[2 * b] = gv;
         e.partials[2 * b + 1] = tv;
@@ -1413,6 +1489,22 @@ __global__ void __launch_bounds__(NT, 2) k_batched_quality(EngineDev e, int64_t 
             e.state[i] = st;
         }
     }
+}
+
+template <int GAUGE, typename R, int NT = 256>
+__global__ void __launch_bounds__(NT, 2) k_batched_quality(EngineDev e, CheckParams cp)
+{
+    quality_block<GAUGE, R, NT>(e, blockIdx.x, cp);
+}
+
+// The check of the instances that have just been folded: idle in most chunks, so a few blocks per SM walk
+// the check's blocks (idle, 16 uneven lattices: 2.6 us instead of 16 us).  A check that is sure to run
+// has one launched block for each: its registers hold the loop less well (MAG 48^4: 472 against 509 us).
+template <int GAUGE, int NT = 256>
+__global__ void __launch_bounds__(NT, 2) k_fold_quality(EngineDev e, int64_t total_blocks, CheckParams cp)
+{
+    if (!any_in_state(e, cp.want_state)) return;
+    for (int64_t b = blockIdx.x; b < total_blocks; b += gridDim.x) quality_block<GAUGE, double, NT>(e, b, cp);
 }
 
 // ---- link-wise kernels over all instances -----------------------------------------------------
@@ -1523,26 +1615,28 @@ __global__ void __launch_bounds__(256) k_export_coulomb(EngineDev e, int i, Rout
 template <typename R, bool TO64>
 __global__ void __launch_bounds__(256) k_reunitarise(EngineDev e, int64_t total_links, int want_state)
 {
-    const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= total_links) return;
-    const int i = find_instance(e.inst, e.ninst, idx, [](const InstDesc &d) { return d.link_begin; });
-    if (e.state[i] != want_state) return;
-    const InstDesc d = e.inst[i];
-    const int64_t l = idx - d.link_begin;
-    const int mu = (int)(l / d.g.V);
-    const int64_t s = l - mu * d.g.V;
-    Link<double> L;
-    load_link_f64<R>(packed_of<R>(d), s, mu, L);
-    project_rows(L);
-    double r[12];
-    pack12(L, r);
-    if (TO64) {
-        packed_of<double>(d).store12(s, mu, r);
-    } else {
-        R o[12];
+    if (!any_in_state(e, want_state)) return;
+    for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total_links;
+         idx += (int64_t)gridDim.x * blockDim.x) {
+        const int i = find_instance(e.inst, e.ninst, idx, [](const InstDesc &d) { return d.link_begin; });
+        if (e.state[i] != want_state) continue;
+        const InstDesc d = e.inst[i];
+        const int64_t l = idx - d.link_begin;
+        const int mu = (int)(l / d.g.V);
+        const int64_t s = l - mu * d.g.V;
+        Link<double> L;
+        load_link_f64<R>(packed_of<R>(d), s, mu, L);
+        project_rows(L);
+        double r[12];
+        pack12(L, r);
+        if (TO64) {
+            packed_of<double>(d).store12(s, mu, r);
+        } else {
+            R o[12];
 #pragma unroll
-        for (int k = 0; k < 12; k++) o[k] = (R)r[k];
-        packed_of<R>(d).store12(s, mu, o);
+            for (int k = 0; k < 12; k++) o[k] = (R)r[k];
+            packed_of<R>(d).store12(s, mu, o);
+        }
     }
 }
 
