@@ -131,6 +131,7 @@ struct gf_ctx {
         e.trace = d_trace;
         e.ntrace = d_ntrace;
         e.trace_cap = trace_cap;
+        e.one = h_inst[0];
         e.stall = d_state + 4 * ninst;
         return e;
     }
@@ -807,34 +808,23 @@ int gf_import(gf_ctx *c, int lat, int real, const void *U, int on_host)
         } else if (c->refine) {
             // Coulomb slice: FP64 master and FP32 working copy, each with W = 1 in its mu = 0 planes
             if (real == GF_FP64) {
-                k_import<double, double><<<blocks, 256, 0, c->stream>>>(c->dev(), i, (const double *)sp);
-                k_import<double, float><<<blocks, 256, 0, c->stream>>>(c->dev(), i, (const double *)sp);
+                k_import<double, double><<<blocks, 256, 0, c->stream>>>(c->dev(), i, (const double *)sp, target);
+                k_import<double, float><<<blocks, 256, 0, c->stream>>>(c->dev(), i, (const double *)sp, target);
             } else {
-                k_import<float, double><<<blocks, 256, 0, c->stream>>>(c->dev(), i, (const float *)sp);
-                k_import<float, float><<<blocks, 256, 0, c->stream>>>(c->dev(), i, (const float *)sp);
+                k_import<float, double><<<blocks, 256, 0, c->stream>>>(c->dev(), i, (const float *)sp, target);
+                k_import<float, float><<<blocks, 256, 0, c->stream>>>(c->dev(), i, (const float *)sp, target);
             }
             c->launches++;
         } else if (target == ST_FP32) {
-            if (real == GF_FP64) k_import<double, float><<<blocks, 256, 0, c->stream>>>(c->dev(), i, (const double *)sp);
-            else k_import<float, float><<<blocks, 256, 0, c->stream>>>(c->dev(), i, (const float *)sp);
+            if (real == GF_FP64) k_import<double, float><<<blocks, 256, 0, c->stream>>>(c->dev(), i, (const double *)sp, target);
+            else k_import<float, float><<<blocks, 256, 0, c->stream>>>(c->dev(), i, (const float *)sp, target);
         } else {
-            if (real == GF_FP64) k_import<double, double><<<blocks, 256, 0, c->stream>>>(c->dev(), i, (const double *)sp);
-            else k_import<float, double><<<blocks, 256, 0, c->stream>>>(c->dev(), i, (const float *)sp);
+            if (real == GF_FP64) k_import<double, double><<<blocks, 256, 0, c->stream>>>(c->dev(), i, (const double *)sp, target);
+            else k_import<float, double><<<blocks, 256, 0, c->stream>>>(c->dev(), i, (const float *)sp, target);
         }
         c->launches++;
         if ((st = launch_status("import"))) return st;
     }
-    const int n = L.count;
-    std::vector<int> states(n, target), stor(n, target == ST_FP32 ? 0 : 1), zeros(n, 0);
-    if ((st = cuda_status(cudaMemcpyAsync(c->d_state + L.first, states.data(), sizeof(int) * n,
-                                          cudaMemcpyHostToDevice, c->stream), "state")) ||
-        (st = cuda_status(cudaMemcpyAsync(c->d_storage + L.first, stor.data(), sizeof(int) * n,
-                                          cudaMemcpyHostToDevice, c->stream), "storage")) ||
-        (st = cuda_status(cudaMemcpyAsync(c->d_sweeps + L.first, zeros.data(), sizeof(int) * n,
-                                          cudaMemcpyHostToDevice, c->stream), "sweeps")) ||
-        (st = cuda_status(cudaMemcpyAsync(c->d_sweeps64 + L.first, zeros.data(), sizeof(int) * n,
-                                          cudaMemcpyHostToDevice, c->stream), "sweeps")))
-        return st;
     return cuda_status(cudaStreamSynchronize(c->stream), "import sync");
 }
 
@@ -1425,6 +1415,7 @@ int gf_autotune(gf_ctx *c, int *choice_fp32, int *choice_fp64)
         EngineDev e = c->dev();
         e.inst = dinst;
         e.state = dstate;
+        e.one = hi[0];
         const int want = prec == 0 ? ST_FP32 : ST_FP64;
         float best = 1e30f;
         int besti = 0;

@@ -44,7 +44,16 @@ struct EngineDev {
     double *trace;        // optional: trace_cap entries of 4 doubles per instance, else null
     int *ntrace;          // per instance: checks recorded (may exceed trace_cap)
     int trace_cap;
+    InstDesc one;         // the first instance's descriptor, by value
 };
+
+// Descriptor of instance i.  A context of one lattice has it in the kernel's parameters: no load of it
+// before the loads of the links, which in a pass of a few microseconds is an L2 round trip of latency.
+__device__ __forceinline__ InstDesc inst_desc(const EngineDev &e, int i)
+{
+    if (e.ninst == 1) return e.one;
+    return e.inst[i];
+}
 
 // Traversal order of a persistent pass: with `reverse` the tiles are walked from the last to the
 // first.  Consecutive parity passes alternate direction, so a pass starts where the previous one
@@ -96,14 +105,18 @@ __global__ void __launch_bounds__(128, MINB) k_batched_pass(EngineDev e, int64_t
     const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (warp >= total_warps) return;
     const int i = find_instance(e.inst, e.ninst, warp, [](const InstDesc &d) { return d.warp_begin; });
-    if (e.state[i] != want_state) return;
-    const InstDesc d = e.inst[i];
+    // one lattice: its state is loaded along with the links and looked at before anything is stored (a
+    // pass is only launched for a precision some instance sweeps in); in a batch, instances that have
+    // dropped out must not cost their links' loads
+    const bool one = e.ninst == 1;
+    if (!one && e.state[i] != want_state) return;
+    const InstDesc d = inst_desc(e, i);
     const PackedField<R> f = packed_of<R>(d);
     AlgoParams pi = p;
     pi.seed = inst_seed(p, i);
     pi.counter = inst_counter(p, i);
     parity_pass_warp<R, GAUGE, ALGO, PackedField<R>, GAUGE == COULOMB, SITE_W>(f, f, d.g, warp - d.warp_begin, parity,
-                                                                               pi, d.w);
+                                                                               pi, d.w, one ? e.state : nullptr, want_state);
 }
 
 // The descriptors and states of the first kInstCache instances, copied into shared memory once per
@@ -121,7 +134,7 @@ __device__ __forceinline__ void fill_inst_cache(const EngineDev &e, InstCache &i
 {
     const int n = e.ninst < kInstCache ? e.ninst : kInstCache;
     if (threadIdx.x < n) {
-        ic.d[threadIdx.x] = e.inst[threadIdx.x];
+        ic.d[threadIdx.x] = inst_desc(e, threadIdx.x);
         ic.state[threadIdx.x] = e.state[threadIdx.x];
     }
     if (threadIdx.x == 0) ic.n = n;
@@ -393,7 +406,7 @@ __global__ void __launch_bounds__(128, MINB) k_batched_pass_pair(EngineDev e, in
     PackedField<R> f{nullptr, 0};
     float2 *W = nullptr;
     if (i >= 0) {
-        const InstDesc &d = e.inst[i];
+        const InstDesc d = inst_desc(e, i);
         ps = pair_site(d, i, tile, parity);
         f = packed_of<R>(d);
         W = d.w;
@@ -657,12 +670,23 @@ __device__ __forceinline__ void store_w(const InstDesc &d, int64_t s, const Link
                 make_float2((float)(W.e[r][k].x - (r == k ? 1.0 : 0.0)), (float)W.e[r][k].y);
 }
 
+// a freshly imported instance: sweeping in its first precision, no sweeps done (written by the import
+// kernel: four small copies from pageable memory per lattice cost about 4 us each)
+__device__ __forceinline__ void reset_instance(const EngineDev &e, int i, int state)
+{
+    e.state[i] = state;
+    e.storage[i] = state == ST_FP64;
+    e.sweeps[i] = 0;
+    e.sweeps64[i] = 0;
+}
+
 // import of a refine instance: FP64 master and FP32 working copy of the links, W = 1
 template <typename Rin>
 __global__ void __launch_bounds__(256) k_import_refine(EngineDev e, int i, const Rin *U)
 {
-    const InstDesc d = e.inst[i];
+    const InstDesc d = inst_desc(e, i);
     const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (idx == 0) reset_instance(e, i, ST_FP32);
     if (idx >= 4 * d.g.V) return;
     const int mu = (int)(idx / d.g.V);
     const int64_t s = idx - mu * d.g.V;
@@ -1415,7 +1439,7 @@ __device__ __forceinline__ void quality_block(const EngineDev &e, int64_t b, con
     // with transitions: the instances sweeping in this precision; without: every instance whose
     // field lives in this precision (uniform over the block)
     if (cp.transitions ? (e.state[i] != cp.want_state) : (e.storage[i] != (sizeof(R) == 8 ? 1 : 0))) return;
-    const InstDesc d = e.inst[i];
+    const InstDesc d = inst_desc(e, i);
     const int64_t lb = b - d.qblock_begin;
     const int64_t s = lb * NT + threadIdx.x;
     double gv = 0, tv = 0;
@@ -1510,10 +1534,11 @@ __global__ void __launch_bounds__(NT, 2) k_fold_quality(EngineDev e, int64_t tot
 // ---- link-wise kernels over all instances -----------------------------------------------------
 // import: reference GpuPattern (rows 0,1) -> packed field of type R
 template <typename Rin, typename R>
-__global__ void __launch_bounds__(256) k_import(EngineDev e, int i, const Rin *U)
+__global__ void __launch_bounds__(256) k_import(EngineDev e, int i, const Rin *U, int state)
 {
-    const InstDesc d = e.inst[i];
+    const InstDesc d = inst_desc(e, i);
     const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (idx == 0) reset_instance(e, i, state);
     if (idx >= 4 * d.g.V) return;
     const int mu = (int)(idx / d.g.V);
     const int64_t s = idx - mu * d.g.V;

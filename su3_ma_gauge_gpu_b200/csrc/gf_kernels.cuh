@@ -22,12 +22,15 @@ __host__ __device__ constexpr double prefactor_gff_dev(int gauge) { return gauge
 // as U_0(t,x) <- W(t,x) U_0(t,x) W(t+1,x)^dagger (the product of the reference's per-sweep left and
 // right multiplications, CoulombKernelsSU3.hxx:226-247), so timeslices share no memory while they
 // sweep.
+// state: where given, the pass leaves the sites alone unless *state is want_state.
 // W columns of the refine mode: float2 planes W[(k*3 + r)*V + s] = W(s)_{r,k}; lane mu < 3 of a
 // site carries column mu through the three subgroup steps (W <- g W), lane 3 carries none.
 template <typename R, int GAUGE, int ALGO, class F, bool TRACK_W = false, bool SITE_W = false>
 __device__ __forceinline__ void parity_pass_warp(const F &Fup, const F &Fdw, const Geom &g, int64_t warp, int parity,
-                                                 const AlgoParams &p, float2 *Wsite = nullptr)
+                                                 const AlgoParams &p, float2 *Wsite = nullptr,
+                                                 const int *state = nullptr, int want_state = 0)
 {
+    const int now = state ? *state : want_state;
     const int lane = threadIdx.x & 31;
     const int mu = lane >> 3;
     const int64_t h = warp * 8 + (lane & 7);
@@ -37,18 +40,22 @@ __device__ __forceinline__ void parity_pass_warp(const F &Fup, const F &Fdw, con
     const bool tdown = (GAUGE == COULOMB) && (mu == 0);
     const bool wlane = TRACK_W && tdown;
     const int64_t sd = tdown ? s : neighbour_down(g, c, mu);
-    Link<R> up, dn;
-    load_link<R>(Fup, s, mu, up);
-    if (wlane) {
+    R ru[12], rd[12];
+    Fup.load12(s, mu, ru);
+    if (wlane) {  // the identity's rows; not stored
 #pragma unroll
-        for (int i = 0; i < 3; i++)
-#pragma unroll
-            for (int j = 0; j < 3; j++) dn.e[i][j] = cx<R>(i == j ? (R)1 : (R)0, (R)0);
+        for (int k = 0; k < 12; k++) rd[k] = (k == 0 || k == 8) ? (R)1 : (R)0;
     } else if (tdown) {
-        load_link<R>(Fdw, sd, mu, dn);
+        Fdw.load12(sd, mu, rd);
     } else {
-        load_link<R>(Fup, sd, mu, dn);
+        Fup.load12(sd, mu, rd);
     }
+    if (now != want_state) return;  // (an instance that is not swept in this precision; warp-uniform)
+    Link<R> up, dn;
+    unpack12(up, ru);
+    reconstruct(up);
+    unpack12(dn, rd);
+    reconstruct(dn);
     Rng<R> rng;
     if (ALGO == ALG_SA || ALGO == ALG_SR || ALGO == ALG_RANDOM) rng.init(ref_rng_tid(h), p.seed, p.counter);
     Cx<R> wcol[3];

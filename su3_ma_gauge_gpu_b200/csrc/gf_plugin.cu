@@ -268,7 +268,9 @@ using namespace gfb;
 struct gf_stats {
     int gauge, real, stop_max, device;
     Geom g;
-    double *scratch;       // partials (2 per block) + result (2)
+    double *scratch;       // partials (2 per block)
+    double *result;        // functional, theta: page-locked host memory the kernel writes directly (a copy
+                           // to the caller's pageable stack would be a second, staged transfer per call)
     unsigned int *ticket;
     unsigned blocks;
 };
@@ -388,13 +390,14 @@ int gf_stats_create(int gauge, int real, const int32_t size[4], int stopping, gf
     s->g = g;
     s->blocks = (unsigned)((g.V + 255) / 256);
     cudaGetDevice(&s->device);
-    st = cuda_status(cudaMalloc(&s->scratch, sizeof(double) * (2 * (size_t)s->blocks + 2) + 256), "cudaMalloc");
+    st = cuda_status(cudaMalloc(&s->scratch, sizeof(double) * 2 * (size_t)s->blocks + 256), "cudaMalloc");
     if (st) {
         delete s;
         return st;
     }
-    s->ticket = (unsigned int *)(s->scratch + 2 * (size_t)s->blocks + 2);
+    s->ticket = (unsigned int *)(s->scratch + 2 * (size_t)s->blocks);
     st = cuda_status(cudaMemset(s->ticket, 0, sizeof(unsigned int)), "cudaMemset");
+    if (!st) st = cuda_status(cudaHostAlloc((void **)&s->result, 2 * sizeof(double), cudaHostAllocMapped), "cudaHostAlloc");
     if (st) {
         cudaFree(s->scratch);
         delete s;
@@ -416,21 +419,20 @@ int gf_stats_generate(gf_stats *s, const void *U, void *stream, double *gff, dou
     a.U = U;
     a.g = s->g;
     a.o.partials = s->scratch;
-    a.o.result = s->scratch + 2 * (size_t)s->blocks;
     a.o.ticket = s->ticket;
     a.o.gff_site = nullptr;
     a.o.theta_site = nullptr;
+    void *result = nullptr;
+    int st = cuda_status(cudaHostGetDevicePointer(&result, s->result, 0), "cudaHostGetDevicePointer");
+    if (st) return st;
+    a.o.result = (double *)result;
     a.stop_max = s->stop_max;
     a.stream = (cudaStream_t)stream;
-    int st = quality_dispatch(s->gauge, a);
-    if (st) return st;
-    double h[2];
-    st = cuda_status(cudaMemcpyAsync(h, a.o.result, sizeof(h), cudaMemcpyDeviceToHost, a.stream), "cudaMemcpyAsync");
-    if (st) return st;
+    if ((st = quality_dispatch(s->gauge, a))) return st;
     st = cuda_status(cudaStreamSynchronize(a.stream), "cudaStreamSynchronize");
     if (st) return st;
-    if (gff) *gff = h[0];
-    if (theta) *theta = h[1];
+    if (gff) *gff = s->result[0];
+    if (theta) *theta = s->result[1];
     return GF_OK;
 }
 
@@ -438,6 +440,7 @@ int gf_stats_destroy(gf_stats *s)
 {
     if (!s) return GF_OK;
     cudaFree(s->scratch);
+    cudaFreeHost(s->result);
     delete s;
     return GF_OK;
 }
