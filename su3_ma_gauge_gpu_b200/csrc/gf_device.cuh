@@ -960,8 +960,8 @@ __device__ __forceinline__ void subgroup_mult2(Link2 &up, Link2 &dn, const float
     }
 }
 
-template <int GAUGE, int ALGO, int I, int J>
-__device__ __forceinline__ void subgroup_step_pair2(Link2 &up, Link2 &dn, int role, const AlgoParams &p, Rng<float> &rng)
+template <int GAUGE, int I, int J>
+__device__ __forceinline__ void subgroup_sum_pair2(const Link2 &up, const Link2 &dn, int role, float w[4])
 {
     Link<float> u[2], d[2];
 #pragma unroll
@@ -969,22 +969,82 @@ __device__ __forceinline__ void subgroup_step_pair2(Link2 &up, Link2 &dn, int ro
         one_of(up, h, u[h]);
         one_of(dn, h, d[h]);
     }
-    float w[4];
     subgroup_sum_pair<GAUGE, I, J>(u, d, role, w);
+}
+template <int GAUGE, int ALGO, int I, int J, bool SITE_W>
+__device__ __forceinline__ void subgroup_step_pair2(Link2 &up, Link2 &dn, int role, const AlgoParams &p,
+                                                    Rng<float> &rng, Cx<float> (*wcol)[3])
+{
+    float w[4];
+    subgroup_sum_pair2<GAUGE, I, J>(up, dn, role, w);
     subgroup_finish<GAUGE, ALGO, 16>(w, p, rng);
     subgroup_mult2<I, J>(up, dn, w);
+    if (SITE_W) left_mult_dcolumn<I, J>(*wcol, w, role);
 }
 
-// site_update_pair for the rules that draw no random numbers, without W
-template <int GAUGE, int ALGO>
-__device__ __forceinline__ void site_update_pair2(Link2 &up, Link2 &dn, int role, const AlgoParams &p)
+// site_update_pair of a lane's links in packed form
+template <int GAUGE, int ALGO, bool SITE_W>
+__device__ __forceinline__ void site_update_pair2(Link2 &up, Link2 &dn, int role, const AlgoParams &p, Rng<float> &rng,
+                                                  Cx<float> (*wcol)[3] = nullptr)
 {
-    static_assert(ALGO == ALG_OR || ALGO == ALG_MICRO, "rules without random numbers");
-    Rng<float> rng;
-    subgroup_step_pair2<GAUGE, ALGO, 0, 2>(up, dn, role, p, rng);
-    subgroup_step_pair2<GAUGE, ALGO, 1, 2>(up, dn, role, p, rng);
-    subgroup_step_pair2<GAUGE, ALGO, 0, 1>(up, dn, role, p, rng);
+    if constexpr (ALGO == ALG_SA) {
+#pragma unroll 1
+        for (int k = 0; k < 3; k++) {
+            float w[4];
+            on_subgroup(k, [&](auto s) { subgroup_sum_pair2<GAUGE, s.I, s.J>(up, dn, role, w); });
+            subgroup_finish<GAUGE, ALGO, 16>(w, p, rng);
+            on_subgroup(k, [&](auto s) {
+                subgroup_mult2<s.I, s.J>(up, dn, w);
+                if (SITE_W) left_mult_dcolumn<s.I, s.J>(*wcol, w, role);
+            });
+        }
+        return;
+    }
+    subgroup_step_pair2<GAUGE, ALGO, 0, 2, SITE_W>(up, dn, role, p, rng, wcol);
+    subgroup_step_pair2<GAUGE, ALGO, 1, 2, SITE_W>(up, dn, role, p, rng, wcol);
+    subgroup_step_pair2<GAUGE, ALGO, 0, 1, SITE_W>(up, dn, role, p, rng, wcol);
 }
+
+// The four links of a lane in the two-lanes-per-site layout: packed in FP32, scalar in FP64.
+template <typename R>
+struct PairLinks {
+    Link<R> up[2], dn[2];
+    __device__ __forceinline__ void set(const R (&ru)[2][12], const R (&rd)[2][12])
+    {
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            unpack12(up[j], ru[j]);
+            unpack12(dn[j], rd[j]);
+            reconstruct(up[j]);
+            reconstruct(dn[j]);
+        }
+    }
+    template <int GAUGE, int ALGO, bool SITE_W>
+    __device__ __forceinline__ void update(int role, const AlgoParams &p, Rng<R> &rng, Cx<R> (*wcol)[3] = nullptr)
+    {
+        site_update_pair<GAUGE, ALGO, R, SITE_W>(up, dn, role, p, rng, wcol);
+    }
+    __device__ __forceinline__ void rows_up(int j, R r[12]) const { pack12(up[j], r); }
+    __device__ __forceinline__ void rows_dn(int j, R r[12]) const { pack12(dn[j], r); }
+};
+template <>
+struct PairLinks<float> {
+    Link2 up, dn;
+    __device__ __forceinline__ void set(const float (&ru)[2][12], const float (&rd)[2][12])
+    {
+        pack_rows(up, ru[0], ru[1]);
+        pack_rows(dn, rd[0], rd[1]);
+        reconstruct2(up);
+        reconstruct2(dn);
+    }
+    template <int GAUGE, int ALGO, bool SITE_W>
+    __device__ __forceinline__ void update(int role, const AlgoParams &p, Rng<float> &rng, Cx<float> (*wcol)[3] = nullptr)
+    {
+        site_update_pair2<GAUGE, ALGO, SITE_W>(up, dn, role, p, rng, wcol);
+    }
+    __device__ __forceinline__ void rows_up(int j, float r[12]) const { unpack_rows(up, j, r); }
+    __device__ __forceinline__ void rows_dn(int j, float r[12]) const { unpack_rows(dn, j, r); }
+};
 
 // ---- lattice geometry -----------------------------------------------------------------------
 // Division by a lattice extent without a divide instruction: for 0 <= n < 2^31 and d >= 1,

@@ -356,7 +356,7 @@ int launch_pass(const gf_ctx *c, const EngineDev &e, const PassArgs &a, const gf
     // The heat bath goes by size, whatever shape OR was tuned to.  With W tracked it stays with the
     // tuned layout: the two layouts round W's columns differently (the links they do not).
     if constexpr (ALGO == ALG_SA) {
-        if (!(sizeof(R) == 4 && c->site_w) && pair_fills(a.c->total_warps, c->num_sms, sizeof(R) == 8))
+        if (!(sizeof(R) == 4 && c->site_w) && pair_fills(a.c->total_warps, c->num_sms, sizeof(R) == 8, true))
             return launch_pair<R, GAUGE, ALGO>(c, e, a);
     }
     return launch_other<R, GAUGE, ALGO>(c, e, a, sh);

@@ -400,8 +400,10 @@ __global__ void __launch_bounds__(128, MINB) k_batched_pass_pair(EngineDev e, in
         if (e.state[i] != want_state) i = -1;
     }
     if (!__any_sync(0xffffffffu, i >= 0)) return;
-    Link<R> up[2], dn[2];
-    Cx<R> wcol[3];
+    // an idle tile's lanes hold links that couple to nothing (they exchange only with each other and store
+    // nothing)
+    R ru[2][12] = {}, rd[2][12] = {};
+    Cx<R> wcol[3] = {};
     PairSite ps{-1, 0, 0, {0, 0}};
     PackedField<R> f{nullptr, 0};
     float2 *W = nullptr;
@@ -412,11 +414,13 @@ __global__ void __launch_bounds__(128, MINB) k_batched_pass_pair(EngineDev e, in
         W = d.w;
 #pragma unroll
         for (int j = 0; j < 2; j++) {
-            load_link<R>(f, ps.s, 2 * role + j, up[j]);
-            if (wlane && j == 0)
-                set_identity(dn[j]);
-            else
-                load_link<R>(f, ps.sd[j], 2 * role + j, dn[j]);
+            f.load12(ps.s, 2 * role + j, ru[j]);
+            if (wlane && j == 0) {  // the identity's rows; not stored
+                rd[j][0] = (R)1;
+                rd[j][8] = (R)1;
+            } else {
+                f.load12(ps.sd[j], 2 * role + j, rd[j]);
+            }
         }
         if (SITE_W) {
 #pragma unroll
@@ -425,25 +429,22 @@ __global__ void __launch_bounds__(128, MINB) k_batched_pass_pair(EngineDev e, in
                 wcol[r] = cx<R>((R)v.x, (R)v.y);
             }
         }
-    } else {  // idle tile: no coupling, so every update leaves the (unstored) links alone
-#pragma unroll
-        for (int j = 0; j < 2; j++)
-#pragma unroll
-            for (int a = 0; a < 3; a++)
-#pragma unroll
-                for (int b = 0; b < 3; b++) up[j].e[a][b] = dn[j].e[a][b] = cx<R>((R)0, (R)0);
-#pragma unroll
-        for (int r = 0; r < 3; r++) wcol[r] = cx<R>((R)0, (R)0);
     }
+    PairLinks<R> links;
+    links.set(ru, rd);
     Rng<R> rng;
     if (ALGO == ALG_SA || ALGO == ALG_SR || ALGO == ALG_RANDOM)
         rng.init(ref_rng_tid(ps.h), inst_seed(p, i < 0 ? 0 : i), inst_counter(p, i < 0 ? 0 : i));
-    site_update_pair<GAUGE, ALGO, R, SITE_W>(up, dn, role, p, rng, &wcol);
+    links.template update<GAUGE, ALGO, SITE_W>(role, p, rng, &wcol);
     if (i < 0) return;
 #pragma unroll
     for (int j = 0; j < 2; j++) {
-        store_link<R>(f, ps.s, 2 * role + j, up[j]);
-        if (!(wlane && j == 0)) store_link<R>(f, ps.sd[j], 2 * role + j, dn[j]);
+        links.rows_up(j, ru[j]);
+        f.store12(ps.s, 2 * role + j, ru[j]);
+        if (!(wlane && j == 0)) {
+            links.rows_dn(j, rd[j]);
+            f.store12(ps.sd[j], 2 * role + j, rd[j]);
+        }
     }
     if (SITE_W) {
 #pragma unroll
@@ -618,7 +619,8 @@ __global__ void __launch_bounds__(128, MINB) k_batched_pass_pair_packed(EngineDe
             pack_rows(dn, cur.dn[0], cur.dn[1]);
             reconstruct2(up);
             reconstruct2(dn);
-            site_update_pair2<GAUGE, ALGO>(up, dn, role, p);
+            Rng<float> rng;  // (these rules draw nothing)
+            site_update_pair2<GAUGE, ALGO, false>(up, dn, role, p, rng);
             if (i >= 0) {
                 const PackedField<float> f = packed_of<float>(inst_at(e, ic, i));
 #pragma unroll

@@ -30,10 +30,14 @@ inline double prefactor_gff(int gauge) { return gauge == GF_COULOMB ? 1.0 / 9.0 
 inline double prefactor_a(int) { return 1.0 / 3.0; }
 
 // Whether a pass over `tiles` 8-site tiles fills the device with two lanes per site; below that, four
-// lanes per site put twice the warps on it.  Landau heat bath, us per pass with four / two lanes: FP64
-// 8^4 (256 tiles) 10.7 / 12.7, 12^4 (1296) 18.1 / 14.7, 16^4 (4096) 33.8 / 25.2; FP32 8^4 8.9 / 10.5,
-// 12^4 10.6 / 11.2, 16^4 19.0 / 15.0.  FP64 is bound by its arithmetic pipe, so fewer warps fill it.
-inline bool pair_fills(int64_t tiles, int sms, bool fp64) { return tiles > (int64_t)sms * (fp64 ? 4 : 16); }
+// lanes per site put twice the warps on it.  us per pass with four / two lanes, Landau: FP32 OR 12^4 (1296
+// tiles) 6.0 / 6.3, 16^4 (4096) 8.4 / 7.4; FP64 OR 12^4 6.5 / 8.4, 16^4 12.5 / 12.5, 32^4 173 / 142; heat
+// bath FP32 8^4 (256) 8.9 / 10.5, 16^4 19.0 / 15.0, FP64 8^4 10.7 / 12.7, 12^4 18.1 / 14.7 -- in FP64 it is
+// bound by the arithmetic pipe, which fewer warps fill.
+inline bool pair_fills(int64_t tiles, int sms, bool fp64, bool heat_bath)
+{
+    return tiles > (int64_t)sms * (fp64 ? (heat_bath ? 4 : 32) : 16);
+}
 
 // compile-time dispatch of a functor over the gauge / algorithm template parameters
 template <template <int, int> class K, typename... Args>

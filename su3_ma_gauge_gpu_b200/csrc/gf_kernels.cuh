@@ -88,140 +88,6 @@ __global__ void __launch_bounds__(128) k_parity_pass(F Fup, F Fdw, Geom g, int p
     parity_pass_warp<R, GAUGE, ALGO>(Fup, Fdw, g, warp, parity, p);
 }
 
-// The same pass as a persistent kernel with register prefetch: each warp walks a strided list of
-// 8-site tiles and loads its lane's two links of the next tile into registers before it updates
-// the current one, so a tile's loads are in flight through the arithmetic of the previous one.
-// Odd parities walk the tiles backwards: a driver that calls parity 0 and then parity 1 finds the
-// links the first pass touched last still in L2.  Same site update and stores as k_parity_pass.
-template <typename R, int GAUGE, int ALGO, class F>
-__global__ void __launch_bounds__(128) k_parity_pass_rp(F Fup, F Fdw, Geom g, int parity, AlgoParams p)
-{
-    const int lane = threadIdx.x & 31, mu = lane >> 3;
-    const bool tdown = (GAUGE == COULOMB) && (mu == 0);  // the temporal down link is in slice t-1
-    const int64_t ntiles = g.Vh / 8;
-    const int64_t stride = (int64_t)gridDim.x * 4;
-    int64_t t = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
-    struct Tile {
-        int64_t h, s, sd;
-        R up[12], dn[12];
-    };
-    auto fetch = [&](int64_t k, Tile &r) {
-        const int64_t tile = parity ? ntiles - 1 - k : k;
-        r.h = tile * 8 + (lane & 7);
-        int32_t c[4];
-        site_coords(g, r.h, parity, c);
-        r.s = r.h + (parity ? g.Vh : 0);
-        r.sd = tdown ? r.s : neighbour_down(g, c, mu);
-        Fup.load12(r.s, mu, r.up);
-        if (tdown)
-            Fdw.load12(r.sd, mu, r.dn);
-        else
-            Fup.load12(r.sd, mu, r.dn);
-    };
-    Tile cur;
-    if (t < ntiles) fetch(t, cur);
-    for (; t < ntiles; t += stride) {  // warp-uniform: every lane of a warp runs the same tiles
-        Tile nxt;
-        if (t + stride < ntiles) fetch(t + stride, nxt);
-        Link<R> up, dn;
-        unpack12(up, cur.up);
-        reconstruct(up);
-        unpack12(dn, cur.dn);
-        reconstruct(dn);
-        Rng<R> rng;
-        if (ALGO == ALG_SA || ALGO == ALG_SR || ALGO == ALG_RANDOM) rng.init(ref_rng_tid(cur.h), p.seed, p.counter);
-        site_update<GAUGE, ALGO>(up, dn, mu, p, rng);
-        store_link<R>(Fup, cur.s, mu, up);
-        if (tdown)
-            store_link<R>(Fdw, cur.sd, mu, dn);
-        else
-            store_link<R>(Fup, cur.sd, mu, dn);
-        cur = nxt;
-    }
-}
-
-// FP64 on the reference layout: the same persistent pass with the next tile staged in shared
-// memory by cp.async instead of registers (the register form holds 200 registers in FP64).  In
-// the reference layout every real of a link is its own plane, so a lane copies its two links as
-// 24 eight-byte chunks; chunk k of a lane sits at [stage][k][lane] (conflict-free), and each lane
-// reads back only what it copied, so its own cp.async.wait_group is the only synchronisation.
-constexpr int kRefStageDoubles = 24;  // two links x rows 0, 1 (12 reals each) per lane
-constexpr size_t ref_staged_smem_bytes(int warps) { return (size_t)warps * 2 * kRefStageDoubles * 32 * 8; }
-
-__device__ __forceinline__ void cp_async8_ref(void *smem, const void *gmem)
-{
-    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem) : "memory");
-}
-
-template <int GAUGE, int ALGO>
-__global__ void __launch_bounds__(128) k_parity_pass_ref_staged(RefField<double> Fup, RefField<double> Fdw, Geom g,
-                                                                int parity, AlgoParams p)
-{
-    extern __shared__ double ref_stage[];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, mu = lane >> 3;
-    const bool tdown = (GAUGE == COULOMB) && (mu == 0);  // the temporal down link is in slice t-1
-    const int64_t ntiles = g.Vh / 8;
-    const int64_t stride = (int64_t)gridDim.x * 4;
-    double *const wbase = ref_stage + (size_t)w * 2 * kRefStageDoubles * 32;  // this warp's two stages
-    struct Tile {
-        int64_t h, s, sd;
-        bool valid;
-    };
-    auto issue = [&](int64_t k, int st) -> Tile {
-        Tile r{0, 0, 0, k < ntiles};
-        if (r.valid) {
-            const int64_t tile = parity ? ntiles - 1 - k : k;
-            r.h = tile * 8 + (lane & 7);
-            int32_t c[4];
-            site_coords(g, r.h, parity, c);
-            r.s = r.h + (parity ? g.Vh : 0);
-            r.sd = tdown ? r.s : neighbour_down(g, c, mu);
-            double *dst = wbase + (size_t)st * kRefStageDoubles * 32;
-            const double *up = Fup.U + (int64_t)mu * 18 * g.V + r.s;
-            const double *dn = (tdown ? Fdw.U : Fup.U) + (int64_t)mu * 18 * g.V + r.sd;
-#pragma unroll
-            for (int q = 0; q < 12; q++) {
-                cp_async8_ref(dst + q * 32 + lane, up + (int64_t)q * g.V);
-                cp_async8_ref(dst + (12 + q) * 32 + lane, dn + (int64_t)q * g.V);
-            }
-        }
-        asm volatile("cp.async.commit_group;\n" ::: "memory");
-        return r;
-    };
-    int64_t t = (int64_t)blockIdx.x * 4 + w;
-    int cur = 0;
-    Tile tc = issue(t, 0);
-    for (; t < ntiles; t += stride) {  // warp-uniform: every lane of a warp runs the same tiles
-        const Tile tn = issue(t + stride, cur ^ 1);
-        asm volatile("cp.async.wait_group 1;\n" ::: "memory");  // this tile's copies have landed
-        const double *src = wbase + (size_t)cur * kRefStageDoubles * 32;
-        double ru[12], rd[12];
-#pragma unroll
-        for (int q = 0; q < 12; q++) {
-            ru[q] = src[q * 32 + lane];
-            rd[q] = src[(12 + q) * 32 + lane];
-        }
-        Link<double> up, dn;
-        unpack12(up, ru);
-        reconstruct(up);
-        unpack12(dn, rd);
-        reconstruct(dn);
-        Rng<double> rng;
-        if (ALGO == ALG_SA || ALGO == ALG_SR || ALGO == ALG_RANDOM) rng.init(ref_rng_tid(tc.h), p.seed, p.counter);
-        site_update<GAUGE, ALGO>(up, dn, mu, p, rng);
-        store_link<double>(Fup, tc.s, mu, up);
-        if (tdown)
-            store_link<double>(Fdw, tc.sd, mu, dn);
-        else
-            store_link<double>(Fup, tc.sd, mu, dn);
-        __syncwarp();  // every lane is done with this stage before the next iteration refills it
-        tc = tn;
-        cur ^= 1;
-    }
-    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-}
-
 // One parity pass over the sites of timeslices [t_begin, t_end) only (4D gauges): in the
 // parity-split order those sites are the contiguous run h in [t_begin Vs/2, t_end Vs/2), so the
 // warps cover that run from its 8-aligned start and leave the sites outside it alone.  A t-slab
@@ -267,9 +133,12 @@ __global__ void __launch_bounds__(128) k_parity_pass_range(F f, Geom g, int pari
 // directions 2 role and 2 role + 1, so the SU(2) update is computed twice per site instead of four
 // times.  Sites outside the range leave their lanes idle, with links that couple to nothing.  Site h
 // draws the random numbers of site h + rng_site_offset.
-// For the heat bath, whose rejection loop costs more than the rest of the update (32^4, one parity,
-// Landau at T = 0.4 / U1xU1 at T = 1: FP32 144 / 234 us against 203 / 6078 us for a lane-wise loop
-// with four lanes per site, FP64 357 / 455 against 387 / 7840 us).
+// All four links of a lane are loaded before any arithmetic (in FP64 one link after the other, each
+// followed by its third row, took 208 us per 32^4 pass with the same 8 warps per SM).  32^4, us per pass,
+// against persistent passes with four lanes per site that looked one tile ahead: OR FP32 67.8 / 78.1 (0.90
+// of the copy peak on 768 B per site update), FP64 142 / 173 (0.87 on 1536 B).  The heat bath, whose
+// rejection loop costs more than the rest of the update, Landau at T = 0.4 / U1xU1 at T = 1: FP32 131 / 219 us
+// against 203 / 6078 us for a lane-wise loop with four lanes per site, FP64 274 / 385 against 387 / 7840 us.
 template <typename R, int GAUGE, int ALGO, class F, int MINB>
 __global__ void __launch_bounds__(128, MINB) k_parity_pass_pair(F Fup, F Fdw, Geom g, int parity, AlgoParams p,
                                                                 int64_t h_lo, int64_t h_hi, int64_t rng_site_offset)
@@ -281,7 +150,7 @@ __global__ void __launch_bounds__(128, MINB) k_parity_pass_pair(F Fup, F Fdw, Ge
     if (!__any_sync(0xffffffffu, active)) return;
     const int64_t s = h + (parity ? g.Vh : 0);
     int64_t sd[2] = {0, 0};
-    Link<R> up[2], dn[2];
+    R ru[2][12] = {}, rd[2][12] = {};
     if (active) {
         int32_t c[4];
         site_coords(g, h, parity, c);
@@ -290,26 +159,24 @@ __global__ void __launch_bounds__(128, MINB) k_parity_pass_pair(F Fup, F Fdw, Ge
             const int mu = 2 * role + j;
             const bool tdown = GAUGE == COULOMB && mu == 0;  // the temporal down link is in slice t-1
             sd[j] = tdown ? s : neighbour_down(g, c, mu);
-            load_link<R>(Fup, s, mu, up[j]);
-            load_link<R>(tdown ? Fdw : Fup, sd[j], mu, dn[j]);
-        }
-    } else {
-#pragma unroll
-        for (int j = 0; j < 2; j++) {
-            set_zero(up[j]);
-            set_zero(dn[j]);
+            Fup.load12(s, mu, ru[j]);
+            (tdown ? Fdw : Fup).load12(sd[j], mu, rd[j]);
         }
     }
+    PairLinks<R> links;
+    links.set(ru, rd);
     Rng<R> rng;
     if (ALGO == ALG_SA || ALGO == ALG_SR || ALGO == ALG_RANDOM)
         rng.init(ref_rng_tid(h + rng_site_offset), p.seed, p.counter);
-    site_update_pair<GAUGE, ALGO, R, false>(up, dn, role, p, rng);
+    links.template update<GAUGE, ALGO, false>(role, p, rng);
     if (!active) return;
 #pragma unroll
     for (int j = 0; j < 2; j++) {
         const int mu = 2 * role + j;
-        store_link<R>(Fup, s, mu, up[j]);
-        store_link<R>(GAUGE == COULOMB && mu == 0 ? Fdw : Fup, sd[j], mu, dn[j]);
+        links.rows_up(j, ru[j]);
+        Fup.store12(s, mu, ru[j]);
+        links.rows_dn(j, rd[j]);
+        (GAUGE == COULOMB && mu == 0 ? Fdw : Fup).store12(sd[j], mu, rd[j]);
     }
 }
 

@@ -81,16 +81,9 @@ struct StepArgs {
 };
 
 // The rules that run with two lanes per site on the reference layout (k_parity_pass_pair) where that
-// fills the device; the others always run with four.  The heat bath in both precisions, and in FP32 the
-// other rules that draw random numbers (32^4: random 80 us per pass against 110 us with four lanes, SR
-// 82 against 106; in FP64 the pass holds 246 registers and is slower, 247 against 238 us).  U1xU1's
-// stochastic and random rules stay with four lanes: there the compiler contracts the two layouts'
-// products differently, everywhere else they agree to the last bit.
-template <typename R>
-constexpr bool pair_rule(int gauge, int algo)
-{
-    return algo == ALG_SA || (sizeof(R) == 4 && (algo == ALG_SR || algo == ALG_RANDOM) && gauge != U1XU1);
-}
+// fills the device (pair_fills).  U1xU1's stochastic and random rules stay with four lanes: there the
+// compiler contracts the two layouts' products differently, everywhere else they agree to the last bit.
+constexpr bool pair_rule(int gauge, int algo) { return !(gauge == U1XU1 && (algo == ALG_SR || algo == ALG_RANDOM)); }
 
 int num_sms()
 {
@@ -117,44 +110,9 @@ struct RefStep {
     {
         RefField<R> fu{(R *)a.U, a.g.V};
         RefField<R> fd{(R *)(a.Udw ? a.Udw : a.U), a.g.V};
-        const int64_t ntiles = a.g.Vh / 8;
-        if constexpr (ALGO == ALG_OR && sizeof(R) == 4) {
-            // FP32 OR, the drivers' hot loop: the persistent register-prefetch pass, one wave of
-            // blocks (0.157 vs 0.160 ms per 32^4 sweep; in FP64 its 200 registers leave 8 warps per
-            // SM and the direct pass is faster, 0.377 vs 0.436 ms)
-            auto kern = k_parity_pass_rp<R, GAUGE, ALGO, RefField<R>>;
-            static int per_sm = 0, sms = 0;  // resident blocks per SM of this instantiation, SMs
-            if (per_sm <= 0) {
-                int dev = 0, o = 0;
-                cudaGetDevice(&dev);
-                cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-                if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, kern, 128, 0) != cudaSuccess || o < 1) o = 1;
-                per_sm = o;
-            }
-            const int64_t need = (ntiles + 3) / 4;
-            const unsigned blocks = (unsigned)std::max<int64_t>(1, std::min<int64_t>(need, (int64_t)sms * per_sm));
-            kern<<<blocks, 128, 0, a.stream>>>(fu, fd, a.g, a.parity, a.p);
-            return launch_status("parity pass (register prefetch)");
-        }
-        if constexpr (ALGO == ALG_OR && sizeof(R) == 8) {
-            // FP64 OR: the persistent pass with the next tile staged by cp.async, one wave of blocks
-            auto kern = k_parity_pass_ref_staged<GAUGE, ALGO>;
-            const size_t smem = ref_staged_smem_bytes(4);  // 48 KB: no opt-in needed
-            static int per_sm = 0, sms = 0;
-            if (per_sm <= 0) {
-                int dev = 0, o = 0;
-                cudaGetDevice(&dev);
-                cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-                if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, kern, 128, smem) != cudaSuccess || o < 1) o = 1;
-                per_sm = o;
-            }
-            const int64_t need = (ntiles + 3) / 4;
-            const unsigned blocks = (unsigned)std::max<int64_t>(1, std::min<int64_t>(need, (int64_t)sms * per_sm));
-            kern<<<blocks, 128, smem, a.stream>>>(fu, fd, a.g, a.parity, a.p);
-            return launch_status("parity pass (cp.async pipelined)");
-        }
-        if constexpr (pair_rule<R>(GAUGE, ALGO)) {
-            if (pair_fills(ntiles, num_sms(), sizeof(R) == 8)) return launch_pair<R, GAUGE, ALGO>(a, 0, a.g.Vh, 0);
+        if constexpr (pair_rule(GAUGE, ALGO)) {
+            if (pair_fills(a.g.Vh / 8, num_sms(), sizeof(R) == 8, ALGO == ALG_SA))
+                return launch_pair<R, GAUGE, ALGO>(a, 0, a.g.Vh, 0);
         }
         const int64_t threads = a.g.Vh * 4;
         const unsigned blocks = (unsigned)((threads + 127) / 128);
@@ -212,8 +170,8 @@ struct RefStepRange {
         } else {
             const int64_t warps = (r.h_hi - (r.h_lo & ~(int64_t)7) + 7) / 8;
             if (warps <= 0) return GF_OK;
-            if constexpr (pair_rule<R>(GAUGE, ALGO)) {
-                if (pair_fills(warps, num_sms(), sizeof(R) == 8))
+            if constexpr (pair_rule(GAUGE, ALGO)) {
+                if (pair_fills(warps, num_sms(), sizeof(R) == 8, ALGO == ALG_SA))
                     return launch_pair<R, GAUGE, ALGO>(r.a, r.h_lo, r.h_hi, r.rng_site_offset);
             }
             RefField<R> fu{(R *)r.a.U, r.a.g.V};
