@@ -65,7 +65,8 @@ def pass_kernel_name(code: int, real: str, refine: bool) -> str:
     if code == 16:
         return f"k_batched_pass_pair<{r}, LANDAU, OR{w}> (two lanes per site)"
     if code == 116:
-        return f"k_batched_pass_pair_rp<{r}, LANDAU, OR{w}> (two lanes per site, register prefetch, persistent)"
+        kernel = f"k_batched_pass_pair_rp<{r}, LANDAU, OR{w}>" if w else "k_batched_pass_pair_packed<LANDAU, OR>"
+        return f"{kernel} (two lanes per site, register prefetch, persistent)"
     if code == 64:
         return f"k_batched_pass<{r}, LANDAU, OR{w}> (64 registers)"
     if code in (2, 4, 8):

@@ -286,7 +286,7 @@ int gf_autotune(gf_ctx *ctx, int *choice_fp32, int *choice_fp64);
  * lanes per site with register prefetch; OR and micro, the other rules run as 6).  GF_COULOMB: 0, 2, 3, 6 or 7;
  * refine FP32: not 1. */
 int gf_set_pass_shape(gf_ctx *ctx, int real, int variant, int warps);
-/* Walk order and occupancy of the persistent passes (variants 1, 3, 7): alternate = 1 walks the
+/* Walk order and occupancy of passes (variants 1, 3, 6, 7): alternate = 1 walks the
  * tiles of every odd-parity pass from the last to the first, so each pass begins on the links the
  * previous pass touched last and still finds them in L2; capped = 1 caps the registers of variants 1
  * (4 warps per block) and 7 so that more warps are resident.  gf_set_pass_shape resets both to 0. */

@@ -101,7 +101,7 @@ struct gf_ctx {
     // tile), `warps` warps per block, grid = num_sms * blocks_per_sm
     struct PassShape {
         int variant = 0, warps = 4, blocks_per_sm = 0;
-        int alternate = 0;  // persistent variants (1, 3, 7): walk the tiles backwards on odd parities
+        int alternate = 0;  // variants 1, 3, 6, 7: walk the tiles backwards on odd parities
         int capped = 0;     // variants 1 (4 warps per block) and 7: registers capped for more resident warps
         int stages = 2;     // variant 1 with 4 warps per block: cp.async stages per warp (2 or 3)
     } shape[2];
@@ -156,7 +156,7 @@ struct PassArgs {
     int parity;
     AlgoParams p;
     int want_state;
-    int reverse;  // persistent passes: walk the tiles backwards
+    int reverse;  // variants 1, 3, 6, 7: walk the tiles backwards
 };
 
 template <typename R, int GAUGE, int ALGO, int WARPS, int MINB = 1, int STAGES = 2>
@@ -255,16 +255,16 @@ int launch_pair(const gf_ctx *c, const EngineDev &e, const PassArgs &a)
         if constexpr (GAUGE != COULOMB) {
             if (c->site_w) {
                 k_batched_pass_pair<R, GAUGE, ALGO, true, 4><<<blocks, 128, 0, a.c->stream>>>(
-                    e, a.c->total_warps, a.parity, a.p, a.want_state);
+                    e, a.c->total_warps, a.parity, a.p, a.want_state, a.reverse);
                 done = true;
             }
         }
         if (!done)
             k_batched_pass_pair<R, GAUGE, ALGO, false, 4><<<blocks, 128, 0, a.c->stream>>>(
-                e, a.c->total_warps, a.parity, a.p, a.want_state);
+                e, a.c->total_warps, a.parity, a.p, a.want_state, a.reverse);
     } else {
         k_batched_pass_pair<R, GAUGE, ALGO, false, 2><<<blocks, 128, 0, a.c->stream>>>(
-            e, a.c->total_warps, a.parity, a.p, a.want_state);
+            e, a.c->total_warps, a.parity, a.p, a.want_state, a.reverse);
     }
     return launch_status("batched parity pass (two lanes per site)");
 }
@@ -1339,18 +1339,18 @@ int gf_autotune(gf_ctx *c, int *choice_fp32, int *choice_fp64)
     // prefetch); pipelined with 2, 4, 8 warps per block; (FP32 only) direct capped at 64 registers and
     // one thread per site (plain and pipelined).  Coulomb passes are direct, register prefetch or two lanes per site; refine-FP32 passes
     // (W tracking) are not the 4-lane pipelined one.
-    static const gf_ctx::PassShape cands64[] = {{0, 4, 0, 0, 0}, {3, 4, 0, 0, 0}, {6, 4, 0, 0, 0},    {1, 4, 0, 1, 0},
+    static const gf_ctx::PassShape cands64[] = {{0, 4, 0, 0, 0}, {6, 4, 0, 1, 0}, {6, 4, 0, 0, 0},    {1, 4, 0, 1, 0},
                                                 {1, 8, 0, 1, 0}, {1, 4, 0, 1, 1}, {3, 4, 0, 1, 0},    {1, 2, 0, 0, 0},
                                                 {1, 4, 0, 0, 0}, {1, 8, 0, 0, 0}, {1, 4, 0, 1, 0, 3}, {1, 4, 0, 0, 0, 3}};
     static const gf_ctx::PassShape cands32[] = {{0, 4, 0, 0, 0}, {2, 4, 0, 0, 0}, {3, 4, 0, 0, 0}, {4, 4, 0, 0, 0},
-                                                {5, 4, 0, 0, 0}, {6, 4, 0, 0, 0}, {7, 4, 0, 0, 0}, {7, 4, 0, 1, 0},
+                                                {5, 4, 0, 0, 0}, {6, 4, 0, 0, 0}, {6, 4, 0, 1, 0}, {7, 4, 0, 1, 0},
                                                 {7, 4, 0, 1, 1}, {3, 4, 0, 1, 0}, {1, 2, 0, 0, 0}, {1, 4, 0, 0, 0},
                                                 {1, 8, 0, 0, 0}};
     // Coulomb slices: direct; register prefetch with and without the alternating walk; two lanes per
     // site (direct, register prefetch with the alternating walk, the same register-capped; the
     // prefetching ones FP32 only, in FP64 they run as the direct one)
     static const gf_ctx::PassShape candsC[] = {{0, 4, 0, 0, 0}, {3, 4, 0, 0, 0}, {3, 4, 0, 1, 0},
-                                               {6, 4, 0, 0, 0}, {7, 4, 0, 1, 0}, {7, 4, 0, 1, 1}};
+                                               {6, 4, 0, 1, 0}, {7, 4, 0, 1, 0}, {7, 4, 0, 1, 1}};
     for (int prec = 0; prec < 2; prec++) {
         if (prec == 0 && !c->mixed) continue;
         const gf_ctx::PassShape *cands = c->gauge == GF_COULOMB ? candsC : prec == 0 ? cands32 : cands64;
@@ -1492,7 +1492,7 @@ int gf_set_pass_shape(gf_ctx *c, int real, int variant, int warps)
     return GF_OK;
 }
 
-// Walk order of the persistent parity passes (variants 1, 3 and 7): alternate = 1 walks the tiles of
+// Walk order of the parity passes of variants 1, 3, 6 and 7: alternate = 1 walks the tiles of
 // odd-parity passes backwards, so every pass starts on the links the previous one touched last;
 // capped = 1 caps the registers of variants 1 (4 warps per block: 128) and 7 (168) so that more
 // warps are resident.

@@ -388,12 +388,15 @@ __device__ __forceinline__ PairSite pair_site(const InstDesc &d, int i, int64_t 
 
 template <typename R, int GAUGE, int ALGO, bool SITE_W, int MINB>
 __global__ void __launch_bounds__(128, MINB) k_batched_pass_pair(EngineDev e, int64_t total_tiles, int parity,
-                                                                 AlgoParams p, int want_state)
+                                                                 AlgoParams p, int want_state, int reverse)
 {
     static_assert(GAUGE != COULOMB || !SITE_W, "Coulomb slices carry W in their temporal planes");
     const int lane = threadIdx.x & 31, role = lane >> 4;
     const bool wlane = GAUGE == COULOMB && role == 0;  // its direction 0 is the slice's W
-    const int64_t tile = (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 2 + ((lane >> 3) & 1);
+    const int64_t npair = (total_tiles + 1) / 2;  // 16-site pair tiles
+    const int64_t pt = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (pt >= npair) return;
+    const int64_t tile = ordered_tile(pt, npair, reverse) * 2 + ((lane >> 3) & 1);
     int i = -1;
     if (tile < total_tiles) {
         i = find_instance(e.inst, e.ninst, tile, [](const InstDesc &d) { return d.warp_begin; });

@@ -151,15 +151,6 @@ __device__ __forceinline__ void load_link(const F &f, int64_t s, int mu, Link<R>
     reconstruct(L);
 }
 
-template <typename R>
-__device__ __forceinline__ void set_zero(Link<R> &L)
-{
-#pragma unroll
-    for (int a = 0; a < 3; a++)
-#pragma unroll
-        for (int b = 0; b < 3; b++) L.e[a][b] = cx<R>((R)0, (R)0);
-}
-
 template <typename R, class F>
 __device__ __forceinline__ void store_link(const F &f, int64_t s, int mu, const Link<R> &L)
 {

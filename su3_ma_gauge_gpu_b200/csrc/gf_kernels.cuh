@@ -104,20 +104,20 @@ __global__ void __launch_bounds__(128) k_parity_pass_range(F f, Geom g, int pari
     const int64_t h = h0 + (lane & 7);
     const bool active = h >= h_lo && h < h_hi;  // the same for the 4 lanes of a site
     int64_t s = 0, sd = 0;
-    Link<R> up, dn;
+    R ru[12] = {}, rd[12] = {};  // (idle lanes: links that couple to nothing and are not stored)
     if (active) {
         int32_t c[4];
         site_coords(g, h, parity, c);
         s = h + (parity ? g.Vh : 0);
         sd = neighbour_down(g, c, mu);
-        load_link<R>(f, s, mu, up);
-        load_link<R>(f, sd, mu, dn);
-    } else {  // no coupling: the update leaves these (unstored) links alone
-#pragma unroll
-        for (int i = 0; i < 3; i++)
-#pragma unroll
-            for (int j = 0; j < 3; j++) up.e[i][j] = dn.e[i][j] = cx<R>((R)0, (R)0);
+        f.load12(s, mu, ru);
+        f.load12(sd, mu, rd);
     }
+    Link<R> up, dn;
+    unpack12(up, ru);
+    reconstruct(up);
+    unpack12(dn, rd);
+    reconstruct(dn);
     Rng<R> rng;
     if (ALGO == ALG_SA || ALGO == ALG_SR || ALGO == ALG_RANDOM)
         rng.init(ref_rng_tid(h + rng_site_offset), p.seed, p.counter);  // the whole lattice's stream for a part of it
@@ -132,20 +132,25 @@ __global__ void __launch_bounds__(128) k_parity_pass_range(F f, Geom g, int pari
 // parity -- the whole of it, or the run of some timeslices: lane role of a site, 0 or 1, holds
 // directions 2 role and 2 role + 1, so the SU(2) update is computed twice per site instead of four
 // times.  Sites outside the range leave their lanes idle, with links that couple to nothing.  Site h
-// draws the random numbers of site h + rng_site_offset.
+// draws the random numbers of site h + rng_site_offset.  Odd parities run from the last site to the first,
+// so the second pass of a sweep begins on the links the first one left in L2.
 // All four links of a lane are loaded before any arithmetic (in FP64 one link after the other, each
 // followed by its third row, took 208 us per 32^4 pass with the same 8 warps per SM).  32^4, us per pass,
-// against persistent passes with four lanes per site that looked one tile ahead: OR FP32 67.8 / 78.1 (0.90
-// of the copy peak on 768 B per site update), FP64 142 / 173 (0.87 on 1536 B).  The heat bath, whose
-// rejection loop costs more than the rest of the update, Landau at T = 0.4 / U1xU1 at T = 1: FP32 131 / 219 us
-// against 203 / 6078 us for a lane-wise loop with four lanes per site, FP64 274 / 385 against 387 / 7840 us.
+// against persistent passes with four lanes per site that looked one tile ahead: OR FP32 61.8 / 78.1 (0.99
+// of the copy peak on 768 B per site update, part of them from L2), FP64 136 / 173 (0.90 on 1536 B); walked
+// forwards in both parities 67.8 and 142.  The heat bath, whose
+// rejection loop costs more than the rest of the update, Landau at T = 0.4 / U1xU1 at T = 1: FP32 127 / 219 us
+// against 203 / 6078 us for a lane-wise loop with four lanes per site, FP64 271 / 385 against 387 / 7840 us.
 template <typename R, int GAUGE, int ALGO, class F, int MINB>
 __global__ void __launch_bounds__(128, MINB) k_parity_pass_pair(F Fup, F Fdw, Geom g, int parity, AlgoParams p,
                                                                 int64_t h_lo, int64_t h_hi, int64_t rng_site_offset)
 {
     const int lane = threadIdx.x & 31, role = lane >> 4;
-    const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int64_t h = (h_lo & ~(int64_t)7) + warp * 16 + (lane & 15);
+    const int64_t h0 = h_lo & ~(int64_t)7, nwarps = (h_hi - h0 + 15) / 16;
+    int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (warp >= nwarps) return;
+    if (parity) warp = nwarps - 1 - warp;
+    const int64_t h = h0 + warp * 16 + (lane & 15);
     const bool active = h >= h_lo && h < h_hi;
     if (!__any_sync(0xffffffffu, active)) return;
     const int64_t s = h + (parity ? g.Vh : 0);
