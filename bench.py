@@ -287,8 +287,8 @@ def reference_gpu_leg(dU_in, gpu_id, fixes) -> dict | None:
 def run_profile_target_sa(nsweeps: int):
     """A short launch sequence of the MAG heat-bath pass for ncu: the MAG 48^4 workload's field
     construction at 32^4 (U = exp(i*0.5*H) under a Haar gauge transform) in a refine context,
-    `nsweeps` SA sweeps at T = 0.7 with the two-lane direct pass (the shape SA runs with when the
-    OR pass is the two-lane register-prefetch one), then with one thread per site."""
+    `nsweeps` SA sweeps at T = 0.7 with the two-lane direct pass (the shape SA runs with when OR is
+    tuned to two lanes per site), then with four lanes per site."""
     import torch
 
     from su3_ma_gauge_gpu_b200 import synthetic as S
@@ -298,7 +298,7 @@ def run_profile_target_sa(nsweeps: int):
     torch.cuda.empty_cache()
     with GaugeFixer([SIZE], gauge="mag", mixed="refine") as gf:
         gf.load(0, dU)
-        for variant in (6, 4):
+        for variant in (6, 0):
             gf.set_pass_shape("fp32", variant, 4)
             gf.sweeps("sa", nsweeps, 0.7, 9, 1)
         g, a = gf.quality()
@@ -315,8 +315,8 @@ def run_profile_target(nsweeps: int, mode: str = "fast"):
     prefetch, register prefetch with alternating walk, the same register-capped); FP64 direct,
     pipelined (alternating walk).
     mode "refine": FP64 master + FP32 working copy with W; FP32 shapes direct, 64-register, register
-    prefetch, thread per site (plain, pipelined), two lanes per site (direct, register prefetch, with
-    alternating walk, the same register-capped); then FP64 direct, pipelined (4 warps; with
+    prefetch, thread per site (plain, pipelined), two lanes per site (direct with alternating walk,
+    register prefetch, with alternating walk, the same register-capped); then FP64 direct, pipelined (4 warps; with
     alternating walk; the same with three cp.async stages), register prefetch.  A third entry in a
     shape is the stage count (gf_set_pass_stages)."""
     import torch
@@ -329,8 +329,8 @@ def run_profile_target(nsweeps: int, mode: str = "fast"):
     if mode == "fast":
         shapes = {"fp32": [(0, 0), (1, 0), (6, 0), (7, 0), (7, 1), (7, 3)], "fp64": [(0, 0), (1, 0), (1, 1)]}
     else:
-        shapes = {"fp32": [(0, 0), (2, 0), (3, 0), (4, 0), (5, 0), (6, 0), (7, 0), (7, 1), (7, 3)],
-                  "fp64": [(0, 0), (1, 0), (1, 1), (1, 1, 3), (3, 0)]}
+        shapes = {"fp32": [(0, 0), (2, 0), (3, 0), (4, 0), (5, 0), (6, 1), (7, 0), (7, 1), (7, 3)],
+                  "fp64": [(0, 0), (1, 0), (1, 1), (1, 1, 3), (3, 0), (6, 1)]}
     with GaugeFixer([SIZE], mixed=True if mode == "fast" else "refine") as gf:
         gf.load(0, dU)
         for real in ("fp32", "fp64"):
