@@ -293,7 +293,7 @@ int gf_set_pass_shape(gf_ctx *ctx, int real, int variant, int warps);
 int gf_set_pass_order(gf_ctx *ctx, int real, int alternate, int capped);
 /* cp.async stages per warp of the pipelined pass (variant 1 with 4 warps per block): 2 (default)
  * keeps the next 8-site tile in flight while the current one is computed, 3 the next two (twice the
- * bytes in flight for the same resident warps; the FP64 pass's choice on a B200).  GF_ERR_INVALID
+ * bytes in flight for the same resident warps).  GF_ERR_INVALID
  * for 3 with any other launch shape; gf_set_pass_shape resets it to 2. */
 int gf_set_pass_stages(gf_ctx *ctx, int real, int stages);
 /* Number of instances (lattices, or timeslices for GF_COULOMB). */

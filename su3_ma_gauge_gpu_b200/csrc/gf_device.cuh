@@ -861,8 +861,9 @@ __device__ __forceinline__ void site_update_thread(Link<R> (&up)[4], Link<R> (&d
 // the two links share float2 registers and every multiply and add of them is one packed instruction
 // (FMUL2 / FFMA2 / FADD2): 39 M instructions per 32^4 pass instead of 53 M.  us per pass, scalar /
 // packed: Coulomb 16 slices of 48^3 116.8 / 104.9, Landau 32^4 in FP32 storage 68.4 / 66.6 (6.05 TB/s).
-// With W tracked (refine mode) it gains nothing, 79.8 / 79.3 (MAG 48^4 393 / 415): there the register
-// cap that buys 12 warps per SM leaves no room for the pairs, so that pass stays scalar.
+// The persistent pass with W tracked gains nothing, 79.8 / 79.3 (MAG 48^4 393 / 415): there the register
+// cap that buys 12 warps per SM leaves no room for the pairs, so it stays scalar; the direct pass with W, which
+// holds no prefetched tile, is packed (87.9 / 78.3, 74.5 with the alternating walk).
 // The products are added in the order the compiler gives the scalar functions
 // above, (fma, product) + (fma, product), so the results are those of the other passes to the last bit.
 struct Link2 {

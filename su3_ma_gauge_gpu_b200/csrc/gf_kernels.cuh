@@ -104,20 +104,20 @@ __global__ void __launch_bounds__(128) k_parity_pass_range(F f, Geom g, int pari
     const int64_t h = h0 + (lane & 7);
     const bool active = h >= h_lo && h < h_hi;  // the same for the 4 lanes of a site
     int64_t s = 0, sd = 0;
-    R ru[12] = {}, rd[12] = {};  // (idle lanes: links that couple to nothing and are not stored)
+    Link<R> up, dn;
     if (active) {
         int32_t c[4];
         site_coords(g, h, parity, c);
         s = h + (parity ? g.Vh : 0);
         sd = neighbour_down(g, c, mu);
-        f.load12(s, mu, ru);
-        f.load12(sd, mu, rd);
+        load_link<R>(f, s, mu, up);
+        load_link<R>(f, sd, mu, dn);
+    } else {  // no coupling: the update leaves these (unstored) links alone
+#pragma unroll
+        for (int i = 0; i < 3; i++)
+#pragma unroll
+            for (int j = 0; j < 3; j++) up.e[i][j] = dn.e[i][j] = cx<R>((R)0, (R)0);
     }
-    Link<R> up, dn;
-    unpack12(up, ru);
-    reconstruct(up);
-    unpack12(dn, rd);
-    reconstruct(dn);
     Rng<R> rng;
     if (ALGO == ALG_SA || ALGO == ALG_SR || ALGO == ALG_RANDOM)
         rng.init(ref_rng_tid(h + rng_site_offset), p.seed, p.counter);  // the whole lattice's stream for a part of it
@@ -139,8 +139,8 @@ __global__ void __launch_bounds__(128) k_parity_pass_range(F f, Geom g, int pari
 // against persistent passes with four lanes per site that looked one tile ahead: OR FP32 61.8 / 78.1 (0.99
 // of the copy peak on 768 B per site update, part of them from L2), FP64 136 / 173 (0.90 on 1536 B); walked
 // forwards in both parities 67.8 and 142.  The heat bath, whose
-// rejection loop costs more than the rest of the update, Landau at T = 0.4 / U1xU1 at T = 1: FP32 127 / 219 us
-// against 203 / 6078 us for a lane-wise loop with four lanes per site, FP64 271 / 385 against 387 / 7840 us.
+// rejection loop costs more than the rest of the update, Landau at T = 0.4 / U1xU1 at T = 1: FP32 128 / 226 us
+// against 203 / 6078 us for a lane-wise loop with four lanes per site, FP64 272 / 380 against 387 / 7840 us.
 template <typename R, int GAUGE, int ALGO, class F, int MINB>
 __global__ void __launch_bounds__(128, MINB) k_parity_pass_pair(F Fup, F Fdw, Geom g, int parity, AlgoParams p,
                                                                 int64_t h_lo, int64_t h_hi, int64_t rng_site_offset)
